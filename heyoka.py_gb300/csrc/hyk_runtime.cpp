@@ -172,6 +172,9 @@ struct KParams {
     uint64_t *inflight;
     uint32_t *serve_status;
     uint64_t idle_ns, max_wait_ns;
+    uint64_t n_slots;
+    uint32_t slot_sms, slot_units;
+    uint32_t slot_layers;
     int persistent;
 };
 
@@ -676,11 +679,35 @@ static void fill_lanes(KParams &k, const hyk_lanes_t *l) {
     k.t_lo = l->time_lo;
 }
 
-// Blocks covering n trajectories: blk of them per block in the lane form,
-// blk / team in the team form.
-static uint64_t lane_blocks(const hyk_module *m, uint64_t n) {
-    const uint64_t per = m->team ? m->blk / m->team : m->blk;
-    return (n + per - 1) / per;
+// Placement of n trajectories (hyk_slot_pos in kernel_common.inc): the grid
+// of the launch, the layers of warps that run and the units of each.
+//
+// One warp per sub-partition (four layers) as long as that holds the batch:
+// the units of each warp are the batch spread evenly over the four layers.
+// Beyond it every resident warp runs, full.  The lane form in double
+// precision stays with one warp per sub-partition up to a quarter more lanes
+// than its first round holds: the lanes behind the slots follow in the places
+// of the first that finish, while a second warp on a sub-partition would halve
+// the speed of both (its FP64 unit is busy 78 % of the time with one warp).
+// A team's recurrences leave the unit idle half of the time with one warp,
+// and float lanes do not use it, so both take more warps at once.
+static uint64_t place(const hyk_module *m, uint64_t n, int ctas_per_sm, KParams &k) {
+    const uint64_t sms = (uint64_t)m->dv->n_sm, wpc = m->blk / 32;
+    const uint64_t units = m->team ? 32 / m->team : 32;
+    const uint64_t all = (uint64_t)ctas_per_sm * wpc, base = std::min<uint64_t>(all, 4);
+    const uint64_t room = base * sms * units;
+    uint64_t layers = all, per = units;
+    if (n <= room) {
+        layers = base;
+        per = std::max<uint64_t>(1, (n + base * sms - 1) / (base * sms));
+    } else if (!m->team && !m->f32 && n <= room + room / 4) {
+        layers = base;
+    }
+    k.slot_sms = (uint32_t)sms;
+    k.slot_units = (uint32_t)per;
+    k.slot_layers = (uint32_t)layers;
+    k.n_slots = sms * layers * per;
+    return sms * ((layers + wpc - 1) / wpc);
 }
 
 // Grid of a launch of f: in global-memory mode every kernel but the
@@ -803,7 +830,8 @@ int hyk_step(hyk_module *m, const hyk_lanes_t *lanes, const double *max_delta_t,
     k.step_oc = outcome;
     k.step_h = h;
     k.step_tc = tc;
-    return launch(m, m->f_step, lane_blocks(m, lanes->n_lanes), m->blk, m->smem, k, stream);
+    const uint64_t grid = place(m, lanes->n_lanes, m->ctas_per_sm, k);
+    return launch(m, m->f_step, grid, m->blk, m->smem, k, stream);
 }
 
 static int fill_prop(hyk_module *m, KParams &k, const hyk_lanes_t *lanes, const hyk_prop_t *p) {
@@ -901,10 +929,7 @@ static int propagate_impl(hyk_module *m, const hyk_lanes_t *lanes, const hyk_pro
         HYK_CU(drv().cuMemsetD32Async((CUdeviceptr)workspace, 0, 4, s));
         k.persistent = 1;
         k.iters_per_launch = p->slice_iters ? p->slice_iters : ~0ULL;
-        // The resident capacity, whatever the number of lanes: a CTA that
-        // finds the queue empty returns at once, and spreading a small batch
-        // over every SM gives each of its warps an FP64 unit of its own.
-        const uint64_t grid = (uint64_t)m->dv->n_sm * (uint64_t)m->ctas_per_sm;
+        const uint64_t grid = place(m, k.n_order, m->ctas_per_sm, k);
         rc = launch(m, m->f_prop, grid, m->blk, m->smem, k, stream);
         if (rc) return rc;
         if (iters) *iters = 1;
@@ -927,13 +952,12 @@ static int propagate_impl(hyk_module *m, const hyk_lanes_t *lanes, const hyk_pro
     k.persistent = 0;
     k.iters_per_launch = 1;
     const bool compact = plain_compacts(m, lanes->n_lanes, workspace_bytes);
-    uint64_t grid = lane_blocks(m, lanes->n_lanes);
+    const uint64_t grid = place(m, lanes->n_lanes, m->ctas_per_sm, k);
     PlainRound chain{compact, check_every, grid, std::min<uint64_t>(4096, (lanes->n_lanes + 255) / 256)};
     if (compact) {
         k.lane_order = reinterpret_cast<uint64_t *>(reinterpret_cast<char *>(workspace) + kWsCounters);
         k.n_order = 0;
         k.act_count = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(workspace) + 12);
-        chain.grid = std::min<uint64_t>(grid, (uint64_t)m->dv->n_sm * (uint64_t)m->ctas_per_sm);
     } else {
         rc = hyk_generic_count_finished(p->status, lanes->n_lanes, k.finished, stream);
         if (rc) return rc;
@@ -1080,7 +1104,7 @@ int hyk_adjoint(hyk_module *m, const hyk_lanes_t *lanes, const double *ck_x, con
     k.queue = reinterpret_cast<uint64_t *>(workspace);
     const CUstream s = (CUstream)stream;
     HYK_CU(drv().cuMemsetD32Async((CUdeviceptr)workspace, 0, 2, s));
-    const uint64_t grid = (uint64_t)m->dv->n_sm * (uint64_t)m->adj_ctas_per_sm;
+    const uint64_t grid = place(m, lanes->n_lanes, m->adj_ctas_per_sm, k);
     return launch(m, m->f_adj, grid, m->blk, m->smem, k, stream);
 }
 
