@@ -293,6 +293,90 @@ struct hyk_module {
     }
 };
 
+// The form of a system for a batch that fills the GPU: 0 = lane form, else the
+// team size.
+//
+// The lane form (one thread per trajectory) needs 32 lanes of
+// coefficients per warp in shared memory and at least 4 resident warps
+// per SM to keep the four FP64 pipes busy.  The team form spreads one
+// trajectory over 2..32 threads: smaller shared memory per warp, at the
+// price of idle threads in the rounds of each dependency level.  The
+// estimate compares busy-thread share x min(1, warps per SM / 4).
+static uint32_t default_team(const hyk::TeamInfo &ti, size_t lane_bytes, size_t real_bytes, const Device &dv) {
+    // Lane form: shared memory with w warps per SM scores min(1, w / 4);
+    // global-memory coefficients (eight warps per SM) score 0.7 (measured:
+    // CR3BP 52 % of the FP64 peak against Kepler's 62 % from shared memory).
+    const size_t warp_bytes = 32 * lane_bytes;
+    uint32_t team = 0;
+    double best = 0.7;
+    if (warp_bytes <= (size_t)dv.smem_optin) {
+        const double w = (double)((size_t)dv.smem_per_sm / (warp_bytes + 1024));
+        best = std::max(best, std::min(1.0, w / 4.0));
+    }
+    for (uint32_t T = 2, l = 1; T <= 32; T *= 2, ++l) {
+        const size_t cta = (size_t)(32 / T) * ti.n_slot * real_bytes;
+        if (cta > (size_t)dv.smem_optin) continue;
+        const double w = (double)((size_t)dv.smem_per_sm / (cta + 1024));
+        const double score = ti.util[l] * std::min(1.0, w / 4.0) * 0.85;
+        if (score > best) {
+            best = score;
+            team = T;
+        }
+    }
+    return team;
+}
+
+// The form for a batch of n trajectories (hyk_config_for), by an estimate of
+// the time of one step of all of them in units of a lane-form step's FP64
+// instructions, 64 cycles each whatever the active lanes of the warp.
+//
+// A team of T threads issues 1 / (T util) of them; a warp alone on its
+// sub-partition takes c times its FP64 time (1.15 measured for the lane form,
+// 1.8 for teams, whose operands come through descriptors), and k warps on one
+// (c^4 + k^4)^(1/4).  A small batch cannot fill the warps of the lane form,
+// so a team that spreads each trajectory wins there: 331 six-body members
+// take 76 us a step with teams of 32 and 99 with 16, 3001 of them 287 and 214
+// (estimated 0.095, 0.127, 0.264, 0.197); 1003 Kepler orbits 58 us in the lane
+// form and 53 with teams of 8.  Lane-form systems so large that their
+// recurrences are split into functions and still spill are counted at c = 4
+// (first-order variational Kepler, 42 equations: 2.05 ms a step in the lane
+// form, 139 us with teams of 32; ptxas 41 s and 0.8 s).  The default form
+// is kept unless another is estimated 5 % faster, and of the teams above the
+// fastest the first within 12 % of it is taken: trajectories of one batch end
+// at different times, and the last ones then run fastest (3001 variational
+// Kepler orbits to t = 10: 47.6 ms with teams of 8, 42.1 with 16).
+// Whole calls, lane form and the choice: 3001 variational Kepler orbits 463 and
+// 42 ms, 331 six-body members (teams of 16 before) 8.1 and 5.0 ms, 1003 Kepler
+// orbits 51.7 and 48.7 ms.
+static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool large, size_t real_bytes, const Device &dv,
+                               uint64_t n) {
+    const double smsp = 4.0 * dv.n_sm;
+    auto cost = [&](double c, double warps, double resident) {
+        const double w = std::ceil(warps / smsp - 1e-9), k = std::max(1.0, std::min(resident, w));
+        const double t = w <= 1.0 ? c : std::pow(c * c * c * c + k * k * k * k, 0.25);
+        return t * std::max(1.0, warps / smsp / k);
+    };
+    double c[6];
+    c[0] = cost(large ? 4.0 : 1.15, (double)n / 32.0, 2.0);
+    for (uint32_t l = 1; l <= 5; ++l) {
+        const uint32_t T = 1u << l;
+        const uint32_t slots = ti.n_slot_cold ? ti.n_slot_cold : ti.n_slot;
+        const size_t cta = (size_t)(32 / T) * slots * real_bytes;
+        c[l] = INFINITY;
+        if (cta > (size_t)dv.smem_optin) continue;
+        const double resident = std::min(24.0, (double)((size_t)dv.smem_per_sm / (cta + 1024))) / 4.0;
+        c[l] = cost(1.8, (double)n * T / 32.0, resident) / (T * ti.util[l]);
+    }
+    const uint32_t dl = dflt ? (uint32_t)__builtin_ctz(dflt) : 0;
+    uint32_t best = 0;
+    for (uint32_t l = 1; l <= 5; ++l)
+        if (c[l] <= c[best]) best = l;
+    if (c[best] * 1.05 >= c[dl]) return dflt;
+    for (uint32_t l = best + 1; best && l <= 5; ++l)
+        if (c[l] <= 1.12 * c[best]) return 1u << l;
+    return best ? 1u << best : 0;
+}
+
 extern "C" {
 
 const char *hyk_last_error(void) { return g_err.c_str(); }
@@ -324,12 +408,6 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     size_t lane_bytes = (size_t)nslot * real_bytes;
     uint32_t blk = m->cfg.block_lanes;
 
-    // Form.  The lane form (one thread per trajectory) needs 32 lanes of
-    // coefficients per warp in shared memory and at least 4 resident warps
-    // per SM to keep the four FP64 pipes busy.  The team form spreads one
-    // trajectory over 2..32 threads: smaller shared memory per warp, at the
-    // price of idle threads in the rounds of each dependency level.  The
-    // estimate compares busy-thread share x min(1, warps per SM / 4).
     hyk::TeamInfo ti;
     std::string terr;
     const bool team_ok = !adjoint && !pin && hyk::team_layout(m->d, order, ti, terr);
@@ -342,25 +420,7 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
                                                  (adjoint ? "adjoint module" : pin ? "pin arithmetic" : terr));
         m->team = want_team;
     } else if (want_team == 0 && team_ok) {
-        // Lane form: shared memory with w warps per SM scores min(1, w / 4);
-        // global-memory coefficients (eight warps per SM) score 0.7 (measured:
-        // CR3BP 52 % of the FP64 peak against Kepler's 62 % from shared memory).
-        const size_t warp_bytes = 32 * lane_bytes;
-        double best = 0.7;
-        if (warp_bytes <= (size_t)dv.smem_optin) {
-            const double w = (double)((size_t)dv.smem_per_sm / (warp_bytes + 1024));
-            best = std::max(best, std::min(1.0, w / 4.0));
-        }
-        for (uint32_t T = 2, l = 1; T <= 32; T *= 2, ++l) {
-            const size_t cta = (size_t)(32 / T) * ti.n_slot * real_bytes;
-            if (cta > (size_t)dv.smem_optin) continue;
-            const double w = (double)((size_t)dv.smem_per_sm / (cta + 1024));
-            const double score = ti.util[l] * std::min(1.0, w / 4.0) * 0.85;
-            if (score > best) {
-                best = score;
-                m->team = T;
-            }
-        }
+        m->team = default_team(ti, lane_bytes, real_bytes, dv);
     }
     if (m->team) {
         if (blk == 0) blk = 32;
@@ -618,6 +678,43 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     }
     if (m->ctas_per_sm < 1) return fail(HYK_ERR_UNSUPPORTED, "the propagation kernel cannot be resident on an SM");
     *out = m.release();
+    return 0;
+}
+
+int hyk_config_for(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t *cfg, int device, uint64_t n_lanes,
+                   hyk_config_t *out) {
+    if (!out) return fail(HYK_ERR_INVALID, "null output pointer");
+    hyk_config_t c{};
+    if (cfg) c = *cfg;
+    *out = c;
+    // What the caller decided stays; single precision (its warps do not share
+    // one slow unit), events, the adjoint, pin arithmetic and the debug build
+    // (whose coefficient checks are the lane form's) keep the default form.
+    const uint32_t fixed = HYK_CFG_PIN_ARITH | HYK_CFG_ADJOINT | HYK_CFG_FLOAT32 | HYK_CFG_GLOBAL_JETS | HYK_CFG_DEBUG;
+    if (n_lanes == 0 || c.team_size || c.block_lanes || c.persist_ctas || (c.flags & fixed)) return 0;
+    hyk::Dec d;
+    std::string err;
+    if (!hyk::load_dec(dd, d, err)) return fail(HYK_ERR_INVALID, err);
+    if (order < 2 || order > 200) return fail(HYK_ERR_INVALID, "the Taylor order must be in [2, 200]");
+    Device *dv = nullptr;
+    const int rc = get_device(device, dv);
+    if (rc) return rc;
+    hyk::TeamInfo ti;
+    if (!hyk::team_layout(d, order, ti, err)) return 0;
+    const size_t lane_bytes = (size_t)hyk::count_slots(d, order) * sizeof(double);
+    const uint32_t dflt = default_team(ti, lane_bytes, sizeof(double), *dv);
+    const bool large = (uint64_t)d.n_ops * order > 3000 || lane_bytes * 32 > (size_t)dv->smem_optin;
+    const uint32_t team = team_for_batch(ti, dflt, large, sizeof(double), *dv, n_lanes);
+    if (team != dflt) c.team_size = team ? team : 1;
+    // A team form whose trajectories are all resident at once without cold
+    // state rows does without them (331 six-body members: teams of 32 87 us a
+    // step with them, 76 without; teams of 16 124 and 99).
+    if (team && ti.n_slot_cold) {
+        const size_t cta = (size_t)(32 / team) * ti.n_slot * sizeof(double);
+        const uint64_t ctas = cta > (size_t)dv->smem_optin ? 0 : std::min<uint64_t>(24, (size_t)dv->smem_per_sm / (cta + 1024));
+        if (n_lanes <= ctas * dv->n_sm * (32 / team)) c.flags |= HYK_CFG_NO_COLD_ROWS;
+    }
+    *out = c;
     return 0;
 }
 

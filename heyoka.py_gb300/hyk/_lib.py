@@ -155,6 +155,7 @@ HYK_SERVE_IDLE, HYK_SERVE_STOP, HYK_SERVE_TIMEOUT = 1, 2, 4
 # Every function the header declares, with its ctypes signature.
 SIGNATURES = {
     "hyk_module_create": (c_int, [P(hyk_decomp_t), c_u32, P(hyk_config_t), c_int, P(c_vp)]),
+    "hyk_config_for": (c_int, [P(hyk_decomp_t), c_u32, P(hyk_config_t), c_int, c_u64, P(hyk_config_t)]),
     "hyk_module_destroy": (c_int, [c_vp]),
     "hyk_module_get_info": (c_int, [c_vp, P(hyk_module_info_t)]),
     "hyk_module_source": (ctypes.c_char_p, [c_vp]),

@@ -129,7 +129,7 @@ def taylor_flow(sys, x0, t_final, pars=None, tol=0.0, t0=0.0):
     dev = x0.device
     if dev.type != "cuda":
         raise ValueError("taylor_flow needs CUDA tensors")
-    fwd = get_module(dec, order, dev.index)
+    fwd = get_module(dec, order, dev.index, n_lanes=x0.shape[1])
     adj = _adjoint_module(dec, order, dev.index)
     B = x0.shape[1]
     f64 = dict(dtype=torch.float64, device=dev)

@@ -238,7 +238,7 @@ def tune_call(ta, call, candidates=DEFAULT_CANDIDATES, repeats=2, apply=True, ve
         cfg = {"team_size": int(T), "global_jets": bool(gj), "block_lanes": int(blk)}
         opts = dict(ta._mod_opts, team_size=int(T), global_jets=bool(gj), block_lanes=int(blk))
         try:
-            m = get_module(ta._dec, ta._order, dev, **opts)
+            m = get_module(ta._dec, ta._order, dev, n_lanes=ta._B, **opts)
         except _lib.HykError as exc:
             trials.append(dict(cfg, skipped=str(exc).splitlines()[0][:160]))
             continue

@@ -23,11 +23,7 @@ class Module:
         L = _lib.load()
         self.dec, self.order, self.device = dec, int(order), int(device)
         self._cdec, self._keep = dec.as_c()
-        flags = (_lib.HYK_CFG_PIN_ARITH if pin_arith else 0) | (_lib.HYK_CFG_HIGH_ACCURACY if high_accuracy else 0)
-        flags |= _lib.HYK_CFG_GLOBAL_JETS if global_jets else 0
-        flags |= _lib.HYK_CFG_FLOAT32 if float32 else 0
-        flags |= 0 if cold_rows else _lib.HYK_CFG_NO_COLD_ROWS
-        flags |= _lib.HYK_CFG_DEBUG if debug else 0
+        flags = _flags(pin_arith, high_accuracy, global_jets, float32, cold_rows, debug)
         self.debug = bool(debug)
         self.float32 = bool(float32)
         cfg = _lib.hyk_config_t(int(block_lanes), int(persist_ctas), flags, int(team_size))
@@ -105,9 +101,44 @@ class Module:
         }
 
 
+def _flags(pin_arith, high_accuracy, global_jets, float32, cold_rows, debug):
+    flags = (_lib.HYK_CFG_PIN_ARITH if pin_arith else 0) | (_lib.HYK_CFG_HIGH_ACCURACY if high_accuracy else 0)
+    flags |= _lib.HYK_CFG_GLOBAL_JETS if global_jets else 0
+    flags |= _lib.HYK_CFG_FLOAT32 if float32 else 0
+    flags |= 0 if cold_rows else _lib.HYK_CFG_NO_COLD_ROWS
+    return flags | (_lib.HYK_CFG_DEBUG if debug else 0)
+
+
+_forms: dict = {}  # (digest, order, device, flags, lanes) -> (team size, flags); bounded
+
+
+def _form_for(dec, order, device, flags, n_lanes):
+    key = (dec.digest(), order, device, flags, n_lanes)
+    r = _forms.get(key)
+    if r is None:
+        cdec, _keep = dec.as_c()
+        cfg, out = _lib.hyk_config_t(0, 0, flags, 0), _lib.hyk_config_t()
+        _lib.check(_lib.load().hyk_config_for(ctypes.byref(cdec), order, ctypes.byref(cfg), device, n_lanes,
+                                              ctypes.byref(out)), "hyk_config_for")
+        r = (int(out.team_size), int(out.flags))
+        with _cache_lock:
+            if len(_forms) >= 1024:
+                _forms.clear()
+            _forms[key] = r
+    return r
+
+
 def get_module(dec: Decomposition, order: int, device: int, block_lanes: int = 0, pin_arith: bool = False,
                team_size: int = 0, persist_ctas: int = 0, high_accuracy: bool = False,
-               global_jets: bool = False, float32: bool = False, cold_rows: bool = True, debug: bool = False) -> Module:
+               global_jets: bool = False, float32: bool = False, cold_rows: bool = True, debug: bool = False,
+               n_lanes: int = 0) -> Module:
+    """The shared module of a system.  ``n_lanes``: the size of the batches it
+    is for (0: unknown, batches that fill the GPU); it selects the kernel form
+    where the other arguments leave it open (``hyk_config_for``)."""
+    if n_lanes and not (team_size or block_lanes or persist_ctas):
+        flags = _flags(pin_arith, high_accuracy, global_jets, float32, cold_rows, debug)
+        team_size, flags = _form_for(dec, int(order), int(device), flags, int(n_lanes))
+        cold_rows = not (flags & _lib.HYK_CFG_NO_COLD_ROWS)
     key = (dec.digest(), int(order), int(device), int(block_lanes), bool(pin_arith), int(team_size), int(persist_ctas),
            bool(high_accuracy), bool(global_jets), bool(float32), bool(cold_rows), bool(debug))
     with _cache_lock:

@@ -205,6 +205,8 @@ def _ensemble(tp, ta, arg, n_iter, gen, **kwargs):
     big = object.__new__(type(ta))
     big.__dict__.update(ta.__dict__)
     big._B = n_iter * B
+    # the kernel form for the whole ensemble, not for one iteration's batch
+    big._mod = ta._module_for(big._B)
     cat = lambda name: torch.cat([getattr(c, name).cpu() for c in copies], dim=-1).to(dev).contiguous()  # noqa: E731
     big._state = cat("_state")
     big._pars = cat("_pars")

@@ -369,7 +369,7 @@ class taylor_adaptive_batch:
                               persist_ctas=int(persist_ctas), high_accuracy=self._high_accuracy,
                               global_jets=bool(global_jets), float32=f32, cold_rows=bool(cold_rows),
                               debug=bool(debug))
-        self._mod = get_module(self._dec, self._order, self._dev, **self._mod_opts)
+        self._mod = get_module(self._dec, self._order, self._dev, n_lanes=B, **self._mod_opts)
         # propagate_grid's own measured choice, when the autotuner found a
         # different one (its modules share the bookkeeping layout)
         self._mod_grid_opts = None
@@ -378,7 +378,7 @@ class taylor_adaptive_batch:
         if bg and (bg["team_size"], bg["global_jets"], bg["block_lanes"]) != (team_size, global_jets, block_lanes):
             self._mod_grid_opts = dict(self._mod_opts, team_size=int(bg["team_size"]),
                                        global_jets=bool(bg["global_jets"]), block_lanes=int(bg["block_lanes"]))
-            self._mod_grid = get_module(self._dec, self._order, self._dev, **self._mod_grid_opts)
+            self._mod_grid = get_module(self._dec, self._order, self._dev, n_lanes=B, **self._mod_grid_opts)
         self._prop_mode = prop_mode
         self._schedule = schedule
         if batch_semantics not in ("reference", "lane"):
@@ -399,6 +399,13 @@ class taylor_adaptive_batch:
         self._final_tc_mask = None  # lanes whose tc must be the final-state jets
         self._launch_events = None
         self._ev = self._ev_alloc(16) if (self._t_events or self._nt_events) else None
+
+    def _module_for(self, n_lanes):
+        """The module for a batch of n_lanes lanes of this integrator's system."""
+        opts = self.__dict__.get("_mod_opts")
+        if opts is None or n_lanes == self._B:
+            return self._mod
+        return get_module(self._dec, self._order, self._dev, n_lanes=n_lanes, **opts)
 
     # ------------------------------------------------------------------ properties
     @property
@@ -1396,9 +1403,10 @@ class taylor_adaptive_batch:
         self.__dict__.setdefault("_nt_events", [])
         self._tdev = dev
         opts = self.__dict__.get("_mod_opts") or dict(high_accuracy=self.__dict__.get("_high_accuracy", False))
-        self._mod = get_module(self._dec, self._order, self._dev, **opts)
+        self._mod = get_module(self._dec, self._order, self._dev, n_lanes=self._B, **opts)
         gopts = self.__dict__.get("_mod_grid_opts")
-        self._mod_grid = None if gopts is None else get_module(self._dec, self._order, self._dev, **gopts)
+        self._mod_grid = None if gopts is None else get_module(self._dec, self._order, self._dev, n_lanes=self._B,
+                                                               **gopts)
 
     def __repr__(self):
         return (

@@ -168,6 +168,15 @@ typedef struct hyk_module_info {
  * (decomposition, order, config). */
 int hyk_module_create(const hyk_decomp_t *d, uint32_t order, const hyk_config_t *cfg, int device,
                       hyk_module **out);
+
+/* The configuration that suits batches of n_lanes trajectories of a system:
+ * *out receives *cfg with the form (team_size, HYK_CFG_NO_COLD_ROWS) filled in
+ * where the caller left it open and another form than the default, which is
+ * made for batches that fill the GPU, is estimated faster for n_lanes.  Every
+ * form gives the same bits.  n_lanes == 0, or a cfg that names a form, a block
+ * size or a CTA count: *out = *cfg. */
+int hyk_config_for(const hyk_decomp_t *d, uint32_t order, const hyk_config_t *cfg, int device, uint64_t n_lanes,
+                   hyk_config_t *out);
 int hyk_module_destroy(hyk_module *m);
 int hyk_module_get_info(const hyk_module *m, hyk_module_info_t *info);
 /* Debug record of a module created with HYK_CFG_DEBUG (HYK_ERR_INVALID for
