@@ -250,6 +250,7 @@ struct Gen {
     std::vector<char> negf, alias, hist, needka;
     std::vector<int> slot, kslot;
     uint32_t nslot = 0, par_slot = 0;
+    uint32_t n_live = 0;  // values of earlier orders the recurrences read
     std::ostringstream o;
     double flops = 0;
 
@@ -315,16 +316,24 @@ struct Gen {
         return v;
     }
 
+    // Histories in registers (inreg): the whole recurrences in one function
+    // whose earlier orders stay in registers, without slots of their own; the
+    // shared memory holds the state rows, the event functions' coefficients
+    // and the parameters.  For systems whose histories fit the registers
+    // (kInreg32, kInreg64 values).
+    bool inreg = false;
+
     // split: one __noinline__ function per order.  Forced for large systems
     // (ptxas time), for the adjoint module and for coefficients in global
     // memory: there a single function of all orders spills (the compiler
     // keeps values of many operations live across the order's long FMA
     // chains), and the per-order functions do not.
     Gen(const Dec &dd, uint32_t order, bool pin_arith, bool adjoint = false, bool cold_rows = false,
-        bool force_split = false)
+        bool force_split = false, bool in_registers = false)
         : d(dd), p(order), N(dd.n_eq), NU(dd.n_u()), pin(pin_arith), adj(adjoint),
           split((uint64_t)dd.n_ops * order > 3000 || adjoint || force_split), evx(!dd.ev.empty()) {
-        coldrows = cold_rows && !adjoint && !evx;
+        inreg = in_registers && !split && !pin_arith;
+        coldrows = cold_rows && !adjoint && !evx && !inreg;
         base.resize(NU);
         negf.assign(NU, 0);
         alias.assign(NU, 0);
@@ -470,18 +479,27 @@ struct Gen {
         // The adjoint module keeps every history up to order p-1.
         const bool ext = adj || evx;
         const uint32_t hl = ext ? p : (p >= 2 ? p - 1 : 1), kl = ext ? p - 1 : (p >= 3 ? p - 2 : 0);
+        n_live = 0;
+        for (uint32_t i = 0; i < N; ++i)
+            if (hread[i]) n_live += p + 1;
         for (uint32_t u = N; u < NU; ++u)
             if (!alias[u] && cst[u]) {
                 hist[u] = 1;  // the order-0 value, read at every order
                 needka[u] = 0;
+                n_live += 1;
+                if (inreg) continue;
                 slot[u] = (int)s;
                 s += 1;
             } else if (hist[u] && !alias[u]) {
+                n_live += hl;
+                if (inreg) continue;
                 slot[u] = (int)s;
                 s += hl;
             }
         for (uint32_t u = 0; u < NU; ++u)
             if (needka[u] && !alias[u] && kl > 0) {
+                n_live += kl;
+                if (inreg) continue;
                 kslot[u] = (int)s;
                 s += kl;
             }
@@ -539,7 +557,7 @@ struct Gen {
 
     // Coefficient of order j of u-variable u (not an alias) while emitting block n.
     std::string ucoef(uint32_t u, uint32_t j, uint32_t n) const {
-        if (j == n) return vname(u, j);
+        if (j == n || inreg) return vname(u, j);
         if (!hist[u] || slot[u] < 0 || (u < N && crow[u] >= 0 && j > 0)) {
             std::fprintf(stderr, "hyk codegen: missing history for u%u\n", u);
             std::abort();
@@ -570,7 +588,7 @@ struct Gen {
             if (cst[r.u]) return "";
             const uint32_t u = (uint32_t)r.u;
             std::string s;
-            if (j == n)
+            if (j == n || inreg)
                 s = kname(u, j);
             else {
                 if (kslot[u] < 0) {
@@ -657,11 +675,11 @@ struct Gen {
 
     void store_hist(uint32_t u, uint32_t n) {
         if (u >= N && cst[u]) {
-            if (n == 0) o << "    " << smem((uint32_t)slot[u]) << " = " << vname(u, 0) << ";\n";
+            if (n == 0 && !inreg) o << "    " << smem((uint32_t)slot[u]) << " = " << vname(u, 0) << ";\n";
             return;
         }
         const uint32_t lim = (adj || evx) ? p : p - 1;  // stored orders: 0..lim-1
-        if (u >= N && hist[u] && n + 1 <= lim) o << "    " << smem((uint32_t)slot[u] + n) << " = " << vname(u, n) << ";\n";
+        if (u >= N && hist[u] && n + 1 <= lim && !inreg) o << "    " << smem((uint32_t)slot[u] + n) << " = " << vname(u, n) << ";\n";
         if (needka[u] && n >= 1) {
             o << "    const hyk_real " << kname(u, n) << " = " << mul(lit((double)n), vname(u, n)) << ";\n";
             flops += 1;
@@ -928,6 +946,7 @@ struct Gen {
         if (!split) {
             o << "static __device__ __noinline__ void hyk_jets(hyk_real *__restrict__ S, const hyk_real t0, "
                  "const unsigned hyk_wm = 0xffffffffu) {\n" << coldg;
+            if (inreg) o << "    HYK_WARP_SYNC();\n";  // reconverge once: nothing is re-read between the orders
             for (uint32_t i = 0; i < N; ++i) o << "    const hyk_real " << vname(i, 0) << " = HYK_SX(" << i << ", 0);\n";
         }
         const uint32_t last = evx ? p : p - 1;  // order p: the event functions' cone only
@@ -979,7 +998,7 @@ struct Gen {
             // different lanes and may have diverged since the last step):
             // hyk_wm names the whole warp, except in the serving kernel, whose
             // idle threads wait elsewhere (hyk_wm 0: the active threads).
-            o << "    HYK_WARP_SYNC();\n";
+            if (!inreg) o << "    HYK_WARP_SYNC();\n";
             if (split) o << "}\n";
         }
         if (split) {
@@ -2109,9 +2128,17 @@ const char *kEvents =
 
 }  // namespace
 
+// Most values of earlier orders the lane form keeps in registers.
+static constexpr uint32_t kInreg32 = 96, kInreg64 = 84;
+
+uint32_t register_values(const Dec &d, uint32_t order, bool f32) {
+    Gen g(d, order, false);
+    return !g.split && g.n_live <= (f32 ? kInreg32 : kInreg64) ? std::max(g.n_live, 1u) : 0;
+}
+
 uint32_t count_slots(const Dec &d, uint32_t order, bool adjoint, bool pin, bool cold_rows, uint32_t *n_cold,
-                     bool split) {
-    Gen g(d, order, pin, adjoint, cold_rows, split);
+                     bool split, bool inreg) {
+    Gen g(d, order, pin, adjoint, cold_rows, split, inreg);
     if (n_cold) *n_cold = g.ncold;
     return g.nslot;
 }
@@ -2123,7 +2150,7 @@ struct PrecisionScope {
 
 bool generate(const Dec &d, uint32_t order, bool pin_arith, uint32_t blk, size_t kparams_size, GenOut &out,
               std::string &err, bool adjoint, uint64_t gmem_stride, bool high_acc, bool f32, uint64_t cold_stride,
-              bool split) {
+              bool split, bool inreg, uint32_t min_ctas) {
     if (order < 2) {
         err = "the Taylor order must be at least 2";
         return false;
@@ -2133,7 +2160,7 @@ bool generate(const Dec &d, uint32_t order, bool pin_arith, uint32_t blk, size_t
         return false;
     }
     PrecisionScope prec(f32);
-    Gen g(d, order, pin_arith, adjoint, cold_stride != 0 && gmem_stride == 0, split);
+    Gen g(d, order, pin_arith, adjoint, cold_stride != 0 && gmem_stride == 0, split, inreg);
     const double p = (double)order;
     const double rhofac = rhofac_of(order);
     std::ostringstream h;
@@ -2154,6 +2181,7 @@ bool generate(const Dec &d, uint32_t order, bool pin_arith, uint32_t blk, size_t
         h << "#define HYK_FMA_ACC(a, b, c) HYK_FMA((a), (b), (c))\n";
         h << "#define HYK_RHO(mp, mq, num) HYK_DM_RHO((mp), (mq), (num), HYK_INV_P, HYK_INV_PM1)\n";
     }
+    h << "#define HYK_LB __launch_bounds__(HYK_TPB" << (g.inreg && min_ctas ? ", " + std::to_string(min_ctas) : "") << ")\n";
     if (adjoint) h << "#define HYK_ADJOINT 1\n";
     h << "#define HYK_HIGH_ACC " << (high_acc ? 1 : 0) << "\n";
     if (g.coldrows) h << "#define HYK_CSTRIDE " << cold_stride << "ULL\n";

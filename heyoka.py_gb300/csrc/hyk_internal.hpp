@@ -37,7 +37,12 @@ struct GenOut {
 // form; implied for the adjoint and for large systems), which keeps the
 // reciprocals of order-0 denominators in slots of their own.
 uint32_t count_slots(const Dec &d, uint32_t order, bool adjoint = false, bool pin = false, bool cold_rows = false,
-                     uint32_t *n_cold = nullptr, bool split = false);
+                     uint32_t *n_cold = nullptr, bool split = false, bool inreg = false);
+
+// The values of earlier orders of a system whose histories the lane form can
+// keep in registers (inreg of count_slots and generate: slots for the state
+// rows, the event coefficients and the parameters only); 0: too many.
+uint32_t register_values(const Dec &d, uint32_t order, bool f32);
 
 // adjoint: also emit the reverse sweep hyk_jets_bw() and the adjoint kernel
 // (and keep every history up to order p-1 for it).
@@ -47,7 +52,8 @@ uint32_t count_slots(const Dec &d, uint32_t order, bool adjoint = false, bool pi
 // stride (the number of threads of the fixed grid).
 bool generate(const Dec &d, uint32_t order, bool pin_arith, uint32_t blk, size_t kparams_size, GenOut &out,
               std::string &err, bool adjoint = false, uint64_t gmem_stride = 0, bool high_acc = false,
-              bool f32 = false, uint64_t cold_stride = 0, bool split = false);
+              bool f32 = false, uint64_t cold_stride = 0, bool split = false, bool inreg = false,
+              uint32_t min_ctas = 0);
 
 // Team form (several threads per trajectory): slot count and the share of
 // busy threads over the rounds of one order for teams of 1, 2, 4, ..., 32.

@@ -422,6 +422,29 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     } else if (want_team == 0 && team_ok) {
         m->team = default_team(ti, lane_bytes, real_bytes, dv);
     }
+    // Lane form of a small system: the histories in registers.  A term of a
+    // convolution then needs no shared-memory loads, which bound the float
+    // kernels (2^20 Kepler orbits, order 9, propagation kernel alone: 3.85 ms
+    // with two CTAs of 256 and the histories in shared memory, 3.34 with them
+    // in registers, 2.86 with the registers held to 80 so that six CTAs of 128
+    // share an SM) and lengthened the step of a warp alone on its FP64 unit
+    // (pendulum, order 20: 26 -> 24 us).
+    const uint32_t n_live = !m->team && !pin && !adjoint && !(m->cfg.flags & HYK_CFG_GLOBAL_JETS)
+                                ? hyk::register_values(m->d, order, f32)
+                                : 0;
+    const bool inreg = n_live != 0;
+    uint32_t min_ctas = 0;
+    if (inreg) {
+        nslot = hyk::count_slots(m->d, order, false, false, false, nullptr, false, true);
+        lane_bytes = (size_t)nslot * real_bytes;
+        if (f32 && blk == 0) {
+            // about 34 registers besides the histories; at most 768 threads an SM
+            blk = 128;
+            const uint32_t regs = (n_live + 34 + 7) / 8 * 8;
+            min_ctas = std::min<uint32_t>(768, 65536 / regs) / blk;
+            min_ctas = std::min<uint32_t>(min_ctas, (uint32_t)((size_t)dv.smem_per_sm / (blk * lane_bytes + 1024)));
+        }
+    }
     if (m->team) {
         if (blk == 0) blk = 32;
         nslot = ti.n_slot;
@@ -511,7 +534,7 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
         // single warp leaves its FP64 pipe idle while that warp waits on
         // shared-memory loads and other latencies; two warps keep it busy.
         uint32_t ncold = 0;
-        const uint32_t cslots = adjoint || !m->d.ev.empty() || (m->cfg.flags & HYK_CFG_NO_COLD_ROWS)
+        const uint32_t cslots = inreg || adjoint || !m->d.ev.empty() || (m->cfg.flags & HYK_CFG_NO_COLD_ROWS)
                                     ? nslot
                                     : hyk::count_slots(m->d, order, adjoint, pin, true, &ncold);
         if (ncold > 0 && cslots < nslot) {
@@ -560,7 +583,7 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
         if (!hyk::generate_team(m->d, order, m->team, blk, sizeof(KParams), g, err, high_acc, f32, m->gmem, m->ncold != 0))
             return fail(HYK_ERR_INVALID, err);
     } else if (!hyk::generate(m->d, order, pin, blk, sizeof(KParams), g, err, adjoint, m->gmem ? m->gmem_threads : 0,
-                              high_acc, f32, m->ncold ? m->cold_threads : 0, m->gmem)) {
+                              high_acc, f32, m->ncold ? m->cold_threads : 0, m->gmem, inreg, min_ctas)) {
         return fail(HYK_ERR_INVALID, err);
     }
     if (g.n_slot != nslot || g.n_cold != m->ncold) return fail(HYK_ERR_INVALID, "internal: slot count mismatch");
