@@ -196,6 +196,19 @@ double powcoef(uint32_t n, uint32_t j, double alpha) {
 }
 
 // The step-size safety factor exp(-2) exp(-0.7 / (p - 1)), as 1/(e e) exp((-7/10)/(p-1)).
+// The packed form of a coefficient for hyk_dm_mulk (kp in the low 20 bits, the
+// exponent's offset and the sign above; |coef| = kp 2^-q, 1024 <= kp < 2048),
+// or 0 when the coefficient has more than 11 significant bits.
+unsigned kpack(double coef) {
+    unsigned long long u;
+    std::memcpy(&u, &coef, sizeof u);
+    const int e = (int)((u >> 52) & 0x7ff) - 1023;
+    if ((u & ((1ULL << 42) - 1)) != 0 || e < -40 || e > 40) return 0;
+    const unsigned kp = 1024u | (unsigned)((u >> 42) & 0x3ffu);
+    const int q = 10 - e;
+    return ((unsigned)(10 - q) << 20) + ((unsigned)(u >> 63) << 31) + kp;
+}
+
 double rhofac_of(uint32_t p) {
     if (g_f32) {
         const float e1 = std::exp(1.0f);
@@ -227,6 +240,7 @@ std::string precision_header(bool pin) {
         h += "#define HYK_MUL(a, b) __fma_rn((a), (b), hyk_nz)\n";
         h += "#define HYK_ADD(a, b) __fma_rn((a), hyk_one, (b))\n";
         h += "#define HYK_SUB(a, b) __fma_rn((b), -hyk_one, (a))\n";
+        h += "#define HYK_MULK(b, k, bad) hyk_dm_mulk((b), (k), (bad))\n";
         h += "#define HYK_DM_EXP hyk_dm_exp\n#define HYK_DM_LOG hyk_dm_log\n#define HYK_DM_SINCOS hyk_dm_sincos\n"
              "#define HYK_DM_POW hyk_dm_pow\n#define HYK_DM_RHO hyk_dm_rho\n";
     }
@@ -821,15 +835,45 @@ struct Gen {
                 keep_inv0(u);
                 break;
             }
-            Acc s{acc};
-            for (uint32_t j = 0; j < n; ++j) {
-                const std::string anj = cf(A, n - j, n);
-                if (anj.empty()) continue;
-                const double coef = powcoef(n, j, alpha);
-                const std::string t = "t" + std::to_string(u) + "_" + std::to_string(n) + "_" + std::to_string(j);
-                o << "    const hyk_real " << t << " = " << mul(lit(coef), anj) << ";\n";
-                flops += 1;
-                term(s, t, ucoef(u, j, n));
+            // The products with the coefficients n alpha - j (alpha + 1): small
+            // half-integers for the usual exponents, formed in integer
+            // arithmetic (hyk_dm_mulk, the same bits) next to the chain, whose
+            // fused multiply-adds leave the other units idle; the chain is
+            // formed again with plain products when an operand was out of the
+            // integer product's range.  (The first term starts the chain and
+            // stays a plain product.)  2^20 Kepler orbits to t = 20: 171 of
+            // 1656 FP64 instructions of a step, propagation kernel 247.0 ->
+            // 227.4 ms.  Not where the recurrences are split into functions: the
+            // CR3BP kernel there waits for its instructions, and the longer code
+            // took 20011 trajectories from 8.55 to 9.68 ms.
+            const std::string bad = "bad" + std::to_string(u) + "_" + std::to_string(n);
+            auto chain = [&](const std::string &name, const std::string &pre, bool ints) {
+                Acc s{name};
+                for (uint32_t j = 0; j < n; ++j) {
+                    const std::string anj = cf(A, n - j, n);
+                    if (anj.empty()) continue;
+                    const double coef = powcoef(n, j, alpha);
+                    const unsigned kp = ints && j > 0 ? kpack(coef) : 0u;
+                    const std::string t = pre + std::to_string(u) + "_" + std::to_string(n) + "_" + std::to_string(j);
+                    o << "    const hyk_real " << t << " = ";
+                    if (kp)
+                        o << "HYK_MULK(" << anj << ", " << kp << "u, " << "&" << bad << ");\n";
+                    else
+                        o << mul(lit(coef), anj) << ";\n";
+                    flops += 1;
+                    term(s, t, ucoef(u, j, n));
+                }
+                return s;
+            };
+            const bool ints = fmaops() && !split && n > 1 && kpack(powcoef(n, 1, alpha)) != 0;
+            if (ints) o << "    unsigned " << bad << " = 0;\n";
+            Acc s = chain(acc, "t", ints);
+            if (ints) {
+                const double f = flops;
+                o << "    if (" << bad << ") {\n";
+                chain("b" + std::to_string(u) + "_" + std::to_string(n), "r", false);
+                o << "    " << acc << " = b" << u << "_" << n << ";\n    }\n";
+                flops = f;
             }
             if (s.first) {
                 def(u, n, z);
@@ -1776,6 +1820,16 @@ struct TeamGen {
         out(u, n0, v);
     }
 
+    // Whether the coefficients n alpha - j (alpha + 1) of a power have the
+    // packed form of hyk_dm_mulk (half-integers of at most 11 bits).
+    bool int_coefs(double alpha) const {
+        if (!g.fmaops()) return false;
+        for (uint32_t n = 2; n <= p; ++n)
+            for (uint32_t j = 1; j < n; ++j)
+                if (!kpack(powcoef(n, j, alpha))) return false;
+        return true;
+    }
+
     void emit_group_op(const Group &gr, bool n0) {
         const uint32_t u = gr.members[0];
         if (!n0 && g.cst[u]) return;  // time-constant: order 0 only
@@ -1961,10 +2015,27 @@ struct TeamGen {
             for (; ai < alphas.size(); ++ai)
                 if (std::memcmp(&alphas[ai], &op.b.num, sizeof(double)) == 0) break;
             const std::string pc = "hyk_pc" + std::to_string(ai) + "[n * (HYK_ORDER + 1)";
-            o << "            hyk_real acc = HYK_MUL(HYK_MUL(" << pc << "], " << at(A, 'a', "n") << "), S[D.c]);\n";
-            o << "#pragma unroll " << ju << "\n";
-            o << "            for (int j = 1; j < n; ++j) acc = " << fma_ << "(HYK_MUL(" << pc << " + j], "
-              << at(A, 'a', "n - j") << "), S[D.c + j], acc);\n";
+            auto chain = [&](bool ints) {
+                o << "            acc = HYK_MUL(HYK_MUL(" << pc << "], " << at(A, 'a', "n") << "), S[D.c]);\n";
+                o << "#pragma unroll " << ju << "\n";
+                o << "            for (int j = 1; j < n; ++j) acc = " << fma_ << "(";
+                if (ints)
+                    o << "HYK_MULK(" << at(A, 'a', "n - j") << ", hyk_pk" << ai << "[n * (HYK_ORDER + 1) + j], &bad)";
+                else
+                    o << "HYK_MUL(" << pc << " + j], " << at(A, 'a', "n - j") << ")";
+                o << ", S[D.c + j], acc);\n";
+            };
+            // (the products in integer arithmetic: see the lane form; 65536
+            // six-body members over a grid 245.7 -> 240.3 ms)
+            const bool ints = int_coefs(op.b.num);
+            o << "            hyk_real acc;\n";
+            if (ints) o << "            unsigned bad = 0;\n";
+            chain(ints);
+            if (ints) {
+                o << "            if (bad) {\n";
+                chain(false);
+                o << "            }\n";
+            }
             out(u, false, "HYK_MUL(HYK_MUL(acc, hyk_invn[n]), S[D.inv])");
             break;
         }
@@ -2080,6 +2151,14 @@ struct TeamGen {
                     const double coef = (j < n) ? powcoef(n, j, alpha) : 0.0;
                     o << " " << lit(coef) << ",";
                 }
+                o << "\n";
+            }
+            o << "};\n";
+            if (!int_coefs(alpha)) continue;
+            o << "static __device__ const unsigned hyk_pk" << ai << "[" << (p + 1) * (p + 1) << "] = {\n";
+            for (uint32_t n = 0; n <= p; ++n) {
+                o << "   ";
+                for (uint32_t j = 0; j <= p; ++j) o << " " << (j > 0 && j < n ? kpack(powcoef(n, j, alpha)) : 0u) << "u,";
                 o << "\n";
             }
             o << "};\n";

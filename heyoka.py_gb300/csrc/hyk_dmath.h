@@ -312,6 +312,29 @@ HYK_DM_FN void hyk_dm_sincos(double x, double *sp, double *cp) {
     }
 }
 
+/* b * coef, rounded to nearest even, in integer arithmetic, for a coefficient
+ * coef = +-kp 2^-q with an integer 1024 <= kp < 2048 (packed by the code generator): the same bits as
+ * the product of the two doubles when b is a normal number whose exponent
+ * leaves the product normal; otherwise *bad becomes non-zero and the result
+ * is meaningless.  No branches, so that the integer units compute it while
+ * the FP64 unit works on other operands (a double product holds that unit
+ * for 64 cycles of a warp, this takes about 22 integer instructions).
+ * k: kp in the low 20 bits, the exponent's and the sign's offset above. */
+HYK_DM_FN double hyk_dm_mulk(double b, unsigned k, unsigned *bad) {
+    const unsigned long long u = HYK_DM_BITS(b);
+    const unsigned hb = (unsigned)(u >> 32), kp = k & 0xfffffu;
+    const unsigned long long p = (unsigned long long)(unsigned)u * kp;
+    const unsigned mh = ((hb & 0xfffffu) | 0x100000u) * kp + (unsigned)(p >> 32);
+    unsigned long long m = ((unsigned long long)mh << 32) | (unsigned)p; /* the exact product, >= 2^62 */
+    const unsigned s = (~mh) >> 31;
+    m <<= s; /* >= 2^63 */
+    const unsigned ml = (unsigned)m;
+    m = (m >> 11) + (((ml & 0x7ffu) + ((ml >> 11) & 1u)) > 0x400u ? 1u : 0u);
+    const unsigned hi = (hb & 0xfff00000u) + (k & 0xfff00000u) - (s << 20) + (unsigned)(m >> 32);
+    *bad |= ((hb & 0x7ff00000u) - (64u << 20)) >= (1900u << 20) ? 1u : 0u;
+    return HYK_DM_FROM(((unsigned long long)hi << 32) | (unsigned)m);
+}
+
 /* x^n for a non-negative integer n by binary powering (fixed product order). */
 HYK_DM_FN double hyk_dm_powi(double x, unsigned n) {
     double r = 1.0, b = x;
