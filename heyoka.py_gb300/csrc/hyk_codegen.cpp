@@ -1481,6 +1481,10 @@ struct TeamGen {
     // multiply-adds, with the operand loads of later terms hoisted; 4 measured
     // best on the 6-body problem against 1, 2 and 8).
     int ju = 4;
+    // Rounds in straight-line code (plan_rounds): the descriptors of a group's
+    // members, one per round of the team, in registers over all orders.
+    uint32_t T = 0;
+    std::map<const Group *, uint32_t> rounds;
 
     TeamGen(const Dec &dd, uint32_t order, bool cold_rows = false)
         : g(dd, order, false, false), d(dd), p(order), N(dd.n_eq), NU(dd.n_u()) {
@@ -1803,8 +1807,8 @@ struct TeamGen {
 
     void out(uint32_t u, bool n0, const std::string &v) {
         o << "            const hyk_real v = " << v << ";\n";
-        o << "            S[D.c" << ((!n0 && g.hist[u]) ? " + n" : "") << "] = v;\n";
-        if (!n0 && g.needka[u]) o << "            S[D.kc + n - 1] = HYK_MUL((hyk_real)n, v);\n";
+        o << "            " << store_if << "S[D.c" << ((!n0 && g.hist[u]) ? " + n" : "") << "] = v;\n";
+        if (!n0 && g.needka[u]) o << "            " << store_if << "S[D.kc + n - 1] = HYK_MUL((hyk_real)n, v);\n";
     }
 
     void addsub(const std::string &a, const std::string &b, bool add, uint32_t u, bool n0) {
@@ -1820,6 +1824,112 @@ struct TeamGen {
         out(u, n0, v);
     }
 
+    // The groups whose rounds are emitted one after the other instead of as a
+    // loop, convolutions first, while their descriptors fit kDescInts registers.
+    // A thread's member of a group is the same at every order: with its
+    // descriptor in registers an order starts its loads at once instead of
+    // after a chain of descriptor loads from global memory (L1), and the rounds of
+    // a group of products run as independent chains.  (At most 112 of the 204 or
+    // 255 registers that eight or ten one-warp CTAs leave a thread; groups of more than
+    // eight rounds stay loops.)  65536 six-body members over a grid, teams of 16:
+    // 240.3 -> 212.4 ms; 331 members, teams of 32: 4.5 -> 4.1 ms; 3001
+    // variational Kepler orbits, teams of 16: 41.3 -> 37.4 ms.
+    static constexpr uint32_t kDescInts = 112;
+    void plan_rounds(uint32_t team) {
+        T = team;
+        struct Cand {
+            const Group *gr;
+            bool conv;
+            uint32_t r, ints;
+        };
+        std::vector<Cand> c;
+        for (auto &lv : levels)
+            for (auto &gr : lv) {
+                const uint32_t u = gr.members[0];
+                if (g.cst[u]) continue;  // order 0 only
+                const auto &op = d.ops[u - N];
+                const Ref A = g.res(op.a), B = g.res(op.b);
+                uint32_t ints = 3;
+                bool conv = true;
+                if (g.fused(u)) {
+                    ints = 3 + (uint32_t)g.fz_x(u).size();
+                    conv = g.fused_sq(u);
+                } else if (op.op == HYK_OP_ADD || op.op == HYK_OP_SUB || op.op == HYK_OP_NEG) {
+                    conv = false;
+                } else if (op.op == HYK_OP_MUL) {
+                    conv = isU(A) && isU(B);
+                } else {
+                    ints = 4;
+                }
+                if (A.kind == HYK_ARG_NUM || B.kind == HYK_ARG_NUM) ints += 2;
+                if (g.needka[u]) ++ints;
+                c.push_back({&gr, conv, ((uint32_t)gr.members.size() + team - 1) / team, ints});
+            }
+        for (auto &gr : supd) c.push_back({&gr, false, ((uint32_t)gr.members.size() + team - 1) / team, 3});
+        uint32_t left = kDescInts;
+        for (const bool conv : {true, false})
+            for (const Cand &x : c)
+                if (x.conv == conv && x.r <= 8 && x.r * x.ints <= left) {
+                    left -= x.r * x.ints;
+                    rounds[x.gr] = x.r;
+                }
+    }
+    std::string dname(const Group &gr, uint32_t c) const { return "d" + std::to_string(gr.off) + "_" + std::to_string(c); }
+    // Whether every thread of the team has a member in round c.
+    bool full_round(const Group &gr, uint32_t c) const { return (c + 1) * T <= gr.members.size(); }
+    std::string member(const Group &gr, uint32_t c) const { return "r + " + std::to_string(c * T); }
+    void load_descs() {
+        auto load = [&](const Group &gr) {
+            auto it = rounds.find(&gr);
+            if (it == rounds.end()) return;
+            for (uint32_t c = 0; c < it->second; ++c) {
+                // (a thread without a member in the last round computes the
+                // group's last one again and stores nothing)
+                const std::string q = member(gr, c), last = std::to_string(gr.members.size() - 1);
+                o << "    const hyk_tdesc " << dname(gr, c) << " = hyk_td[" << gr.off << " + "
+                  << (full_round(gr, c) ? q : "(" + q + " < " + last + " ? " + q + " : " + last + ")") << "];\n";
+            }
+        };
+        for (auto &lv : levels)
+            for (auto &gr : lv) load(gr);
+        for (auto &gr : supd) load(gr);
+    }
+    // Runs body(c) per round with D as that round's descriptor; store guards
+    // the stores of a round that not every thread takes part in.
+    std::string store_if;
+    template <typename F> void per_round(const Group &gr, F body) {
+        const uint32_t R = rounds.at(&gr);
+        for (uint32_t c = 0; c < R; ++c) {
+            o << "        {\n            const hyk_tdesc &D = " << dname(gr, c) << ";\n";
+            store_if = full_round(gr, c) ? "" : "if (" + member(gr, c) + " < " + std::to_string(gr.members.size()) + ") ";
+            body(c);
+            store_if.clear();
+            o << "        }\n";
+        }
+    }
+    // The rounds' convolutions in one loop over j: independent chains, whose
+    // loads wait while another chain's multiply-add is in the FP64 unit.
+    // (acc of round c: acc_c; x and y give the factors of term J.)
+    static std::string with(std::string s, const std::string &from, const std::string &to) {
+        for (size_t k = 0; (k = s.find(from, k)) != std::string::npos; k += to.size()) s.replace(k, from.size(), to);
+        return s;
+    }
+    std::string in_round(const Group &gr, uint32_t c, const std::string &s) const { return with(s, "D.", dname(gr, c) + "."); }
+    void merged_mul(const Group &gr, const Ref &A, const Ref &B) {
+        const uint32_t R = rounds.at(&gr);
+        o << "        {\n";
+        for (uint32_t c = 0; c < R; ++c)
+            o << "            hyk_real acc" << c << " = HYK_MUL(" << in_round(gr, c, at(A, 'a', "0")) << ", "
+              << in_round(gr, c, at(B, 'b', "n")) << ");\n";
+        o << "#pragma unroll " << (R > 1 ? 2 : ju) << "\n            for (int j = 1; j <= n; ++j) {\n";
+        for (uint32_t c = 0; c < R; ++c)
+            o << "                acc" << c << " = HYK_FMA(" << in_round(gr, c, at(A, 'a', "j")) << ", "
+              << in_round(gr, c, at(B, 'b', "n - j")) << ", acc" << c << ");\n";
+        o << "            }\n";
+        per_round(gr, [&](uint32_t c) { out(gr.members[0], false, "acc" + std::to_string(c)); });
+        o << "        }\n";
+    }
+
     // Whether the coefficients n alpha - j (alpha + 1) of a power have the
     // packed form of hyk_dm_mulk (half-integers of at most 11 bits).
     bool int_coefs(double alpha) const {
@@ -1833,14 +1943,29 @@ struct TeamGen {
     void emit_group_op(const Group &gr, bool n0) {
         const uint32_t u = gr.members[0];
         if (!n0 && g.cst[u]) return;  // time-constant: order 0 only
+        const auto AB = opnds(u);
+        o << "        // " << gr.key << "\n";
+        if (!n0 && rounds.count(&gr)) {
+            if (!g.fused(u) && d.ops[u - N].op == HYK_OP_MUL && isU(AB.first) && isU(AB.second))
+                merged_mul(gr, AB.first, AB.second);
+            else
+                per_round(gr, [&](uint32_t) { emit_member(gr, false); });
+            return;
+        }
+        o << "#pragma unroll 1\n";
+        o << "        for (int q = r; q < " << gr.members.size() << "; q += HYK_TEAM) {\n";
+        o << "            const hyk_tdesc &D = hyk_td[" << gr.off << " + q];\n";
+        emit_member(gr, n0);
+        o << "        }\n";
+    }
+
+    // The operation of one member of a group (descriptor D), order n or 0.
+    void emit_member(const Group &gr, bool n0) {
+        const uint32_t u = gr.members[0];
         const auto &op = d.ops[u - N];
         const auto AB = opnds(u);
         const Ref A = AB.first, B = AB.second;
         const std::string fma_ = "HYK_FMA";
-        o << "        // " << gr.key << "\n";
-        o << "#pragma unroll 1\n";
-        o << "        for (int q = r; q < " << gr.members.size() << "; q += HYK_TEAM) {\n";
-        o << "            const hyk_tdesc &D = hyk_td[" << gr.off << " + q];\n";
         if (g.fused_sc(u)) {
             // a + sum_i k_i t_i in one chain (hyk_fuse.h), the lane form's
             // arithmetic; the leaves' slots are in D.b, D.inv, D.prt, D.x3,
@@ -1854,7 +1979,6 @@ struct TeamGen {
                 r = r.empty() ? "HYK_MUL(" + k + ", " + x + ")" : fma_ + "(" + k + ", " + x + ", " + r + ")";
             }
             out(u, n0, r);
-            o << "        }\n";
             return;
         }
         if (g.fused(u)) {
@@ -1890,7 +2014,6 @@ struct TeamGen {
                 o << "            }\n";
                 out(u, false, "acc");
             }
-            o << "        }\n";
             return;
         }
         if (n0) {
@@ -1928,7 +2051,6 @@ struct TeamGen {
                 }
                 break;
             }
-            o << "        }\n";
             return;
         }
         switch (op.op) {
@@ -2075,16 +2197,24 @@ struct TeamGen {
             out(u, false, op.op == HYK_OP_SIN ? "HYK_MUL(acc, hyk_invn[n])" : "(-HYK_MUL(acc, hyk_invn[n]))");
             break;
         }
-        o << "        }\n";
     }
 
     void emit_group_upd(const Group &gr, bool n0) {
-        const uint32_t i = gr.members[0];
-        const Ref R = g.res(d.rhs[i]);
         o << "        // " << gr.key << "\n";
+        if (!n0 && rounds.count(&gr)) {
+            per_round(gr, [&](uint32_t) { emit_upd(gr, false); });
+            return;
+        }
         o << "#pragma unroll 1\n";
         o << "        for (int q = r; q < " << gr.members.size() << "; q += HYK_TEAM) {\n";
         o << "            const hyk_tdesc &D = hyk_td[" << gr.off << " + q];\n";
+        emit_upd(gr, n0);
+        o << "        }\n";
+    }
+
+    void emit_upd(const Group &gr, bool n0) {
+        const uint32_t i = gr.members[0];
+        const Ref R = g.res(d.rhs[i]);
         std::string f;
         if (n0) {
             f = cur(R, 'a', true);
@@ -2103,18 +2233,17 @@ struct TeamGen {
             v = "HYK_MUL(" + f + ", hyk_invn[" + nn + "])";
         o << "            const hyk_real v = " << v << ";\n";
         if (cold) {
-            o << "            S[D.c + " << (n0 ? "1" : "((n + 1) & 1)") << "] = v;\n";
-            o << "            HYK_CROW(D.b, " << nn << ") = v;\n";
+            o << "            " << store_if << "S[D.c + " << (n0 ? "1" : "((n + 1) & 1)") << "] = v;\n";
+            o << "            " << store_if << "HYK_CROW(D.b, " << nn << ") = v;\n";
         } else {
-            o << "            S[D.c + " << nn << "] = v;\n";
+            o << "            " << store_if << "S[D.c + " << nn << "] = v;\n";
         }
         if (g.needka[i]) {
             if (n0)
-                o << "            if (1 < HYK_ORDER) S[D.kc] = " << lit(1.0) << " * v;\n";
+                o << "            if (1 < HYK_ORDER) " << store_if << "S[D.kc] = " << lit(1.0) << " * v;\n";
             else
-                o << "            if (n + 1 < HYK_ORDER) S[D.kc + n] = HYK_MUL((hyk_real)(n + 1), v);\n";
+                o << "            if (n + 1 < HYK_ORDER) " << store_if << "S[D.kc + n] = HYK_MUL((hyk_real)(n + 1), v);\n";
         }
-        o << "        }\n";
     }
 
     void emit_order(bool n0) {
@@ -2173,6 +2302,7 @@ struct TeamGen {
             o << "    for (int i = r; i < HYK_NEQ; i += HYK_TEAM) S[i * HYK_XS] = HYK_CROW(i, 0);\n";
             o << "    __syncwarp();\n";
         }
+        load_descs();
         o << "    {\n        // ---- order 0\n";
         emit_order(true);
         o << "    }\n";
@@ -2326,6 +2456,7 @@ bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, si
         return false;
     }
     tg.g.emit_jets();  // flop count of the same recurrences
+    tg.plan_rounds(team);
     const double p = (double)order;
     const double rhofac = rhofac_of(order);
     const uint32_t nt = tg.nslot | 1u;
@@ -2392,6 +2523,7 @@ bool generate_host(const Dec &d, uint32_t order, bool adjoint, std::string &src,
         else
             h << "#define HYK_SX(i, n) S[(i) * HYK_XS + (n)]\n";
         h << "#define HYK_PAR(k) S[HYK_PAR_SLOT + (k)]\n";
+        tg.plan_rounds(1);
         tg.emit();
         h << tg.o.str();
         h << "extern \"C\" int hyk_host_nslot(void) { return HYK_NSLOT; }\n";
