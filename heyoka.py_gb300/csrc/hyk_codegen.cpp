@@ -2352,6 +2352,13 @@ uint32_t count_slots(const Dec &d, uint32_t order, bool adjoint, bool pin, bool 
     return g.nslot;
 }
 
+// The step-size rule's rho: of one logarithm in double precision, with the
+// same bits as hyk_dm_rho (hyk_rho_one in kernel_common.inc).
+static std::string rho_macro(bool f32) {
+    if (f32) return "#define HYK_RHO(mp, mq, num) HYK_DM_RHO((mp), (mq), (num), HYK_INV_P, HYK_INV_PM1)\n";
+    return "#define HYK_RHO_ONE 1\n#define HYK_RHO(mp, mq, num) hyk_rho_one((mp), (mq), (num))\n";
+}
+
 struct PrecisionScope {
     explicit PrecisionScope(bool f32) { g_f32 = f32; }
     ~PrecisionScope() { g_f32 = false; }
@@ -2388,7 +2395,7 @@ bool generate(const Dec &d, uint32_t order, bool pin_arith, uint32_t blk, size_t
              "? 1.0 / pow((mq) / (num), HYK_INV_PM1) : 1.0 / pow((mp) / (num), HYK_INV_P))\n";
     } else {
         h << "#define HYK_FMA_ACC(a, b, c) HYK_FMA((a), (b), (c))\n";
-        h << "#define HYK_RHO(mp, mq, num) HYK_DM_RHO((mp), (mq), (num), HYK_INV_P, HYK_INV_PM1)\n";
+        h << rho_macro(f32);
     }
     h << "#define HYK_LB __launch_bounds__(HYK_TPB" << (g.inreg && min_ctas ? ", " + std::to_string(min_ctas) : "") << ")\n";
     if (adjoint) h << "#define HYK_ADJOINT 1\n";
@@ -2471,7 +2478,7 @@ bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, si
       << lit(recip(p - 1.0)) << "\n";
     h << precision_header(false);
     h << "#define HYK_FMA_ACC(a, b, c) HYK_FMA((a), (b), (c))\n";
-    h << "#define HYK_RHO(mp, mq, num) HYK_DM_RHO((mp), (mq), (num), HYK_INV_P, HYK_INV_PM1)\n";
+    h << rho_macro(f32);
     h << "#define HYK_NEV 0\n#define HYK_NTEV 0\n#define HYK_HIGH_ACC " << (high_acc ? 1 : 0) << "\n";
     h << kDmath << "\n";
     h << kCommon << "\n";
