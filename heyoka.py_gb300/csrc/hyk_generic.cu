@@ -32,6 +32,59 @@ __global__ void dense_eval_kernel(const R *__restrict__ tc, uint32_t n_eq, uint3
     }
 }
 
+// Continuous output at n_rows times per lane (t, out: row-major over lanes): the
+// step that holds t (the last one that starts at or before it, the first or the
+// last one outside the range, by binary search over the lane's step times),
+// the offset from its start in double length, and Horner's rule on its
+// coefficients where they are stored.  One thread per (row, variable, lane):
+// consecutive lanes read consecutive numbers while they are in the same
+// step.  It replaces, per row, a search, a gather of the step's coefficients
+// into a new array and an evaluation (6 launches a row; 2003 Kepler orbits to
+// t = 6 with 16 rows evaluated, with the larger first store of the records:
+// 13.2 -> 7.5 ms, of which 6.1 are the propagation).
+template <typename R>
+__global__ void coutput_eval_kernel(const R *__restrict__ tcs, const R *__restrict__ thi, const R *__restrict__ tlo,
+                                    uint64_t n_steps, uint32_t n_eq, uint32_t order, uint64_t n_lanes,
+                                    const R *__restrict__ t, R *__restrict__ out) {
+    const uint64_t lane = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (lane >= n_lanes) return;
+    const uint32_t i = blockIdx.y;
+    const uint64_t row = blockIdx.z;
+    const R sgn = thi[n_steps * n_lanes + lane] < thi[lane] ? R(-1) : R(1);
+    const R tv = t[row * n_lanes + lane], key = tv * sgn;
+    // the number of step starts that are not after the key (a not-a-number
+    // key is after all of them)
+    uint64_t lo = 0, hi = n_steps;
+    while (lo < hi) {
+        const uint64_t mid = (lo + hi) / 2;
+        if (!(thi[mid * n_lanes + lane] * sgn > key)) lo = mid + 1;
+        else hi = mid;
+    }
+    const uint64_t k = lo > 0 ? lo - 1 : 0;
+    const R bh = thi[k * n_lanes + lane], bl = tlo[k * n_lanes + lane];
+    const R s = tv + (-bh), bb = s - tv;
+    R e = (tv - (s - bb)) + ((-bh) - bb);
+    e = e + (R(0) - bl);
+    const R dt = s + e;
+    const R *c = tcs + ((k * n_eq + i) * (order + 1)) * n_lanes + lane;
+    R acc = c[(uint64_t)order * n_lanes];
+    for (int n = (int)order - 1; n >= 0; --n) acc = fma_rn(acc, dt, c[(uint64_t)n * n_lanes]);
+    out[(row * n_eq + i) * n_lanes + lane] = acc;
+}
+
+template <typename R>
+int coutput_eval(const R *tcs, const R *thi, const R *tlo, uint64_t n_steps, uint32_t n_eq, uint32_t order,
+                 uint64_t n_lanes, const R *t, uint64_t n_rows, R *out, cudaStream_t s) {
+    const uint64_t blocks = (n_lanes + 127) / 128;
+    if (blocks > 0x7fffffffULL || n_eq > 65535u) return (int)cudaErrorInvalidConfiguration;
+    for (uint64_t r = 0; r < n_rows; r += 65535) {  // (gridDim.z)
+        const unsigned nz = (unsigned)(n_rows - r < 65535 ? n_rows - r : 65535);
+        coutput_eval_kernel<R><<<dim3((unsigned)blocks, n_eq, nz), 128, 0, s>>>(tcs, thi, tlo, n_steps, n_eq, order, n_lanes,
+                                                                               t + r * n_lanes, out + r * n_eq * n_lanes);
+    }
+    return (int)cudaGetLastError();
+}
+
 __global__ void count_finished_kernel(const uint32_t *__restrict__ status, uint64_t n_lanes, uint32_t *finished) {
     uint32_t c = 0;
     for (uint64_t l = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; l < n_lanes; l += (uint64_t)gridDim.x * blockDim.x)
@@ -107,6 +160,17 @@ extern "C" int hyk_generic_dense_eval_f32(const float *tc, uint32_t n_eq, uint32
     const uint64_t grid = (n_lanes + blk - 1) / blk;
     dense_eval_kernel<float><<<(unsigned)grid, blk, 0, (cudaStream_t)stream>>>(tc, n_eq, order, n_lanes, ld, dt, out);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+extern "C" int hyk_generic_coutput_eval(int f32, const void *tcs, const void *thi, const void *tlo, uint64_t n_steps,
+                                        uint32_t n_eq, uint32_t order, uint64_t n_lanes, const void *t, uint64_t n_rows,
+                                        void *out, void *stream) {
+    const cudaStream_t s = (cudaStream_t)stream;
+    const int rc = f32 ? coutput_eval((const float *)tcs, (const float *)thi, (const float *)tlo, n_steps, n_eq, order,
+                                      n_lanes, (const float *)t, n_rows, (float *)out, s)
+                       : coutput_eval((const double *)tcs, (const double *)thi, (const double *)tlo, n_steps, n_eq, order,
+                                      n_lanes, (const double *)t, n_rows, (double *)out, s);
+    return rc == (int)cudaSuccess ? 0 : -2;
 }
 
 extern "C" int hyk_generic_dmath(int fn, const double *x, const double *a, double *out, uint64_t n, void *stream) {

@@ -53,6 +53,9 @@ extern "C" int hyk_generic_dense_eval(const double *tc, uint32_t n_eq, uint32_t 
                                       const double *dt, double *out, void *stream);
 extern "C" int hyk_generic_dense_eval_f32(const float *tc, uint32_t n_eq, uint32_t order, uint64_t n_lanes,
                                           uint64_t ld, const float *dt, float *out, void *stream);
+extern "C" int hyk_generic_coutput_eval(int f32, const void *tcs, const void *thi, const void *tlo, uint64_t n_steps,
+                                        uint32_t n_eq, uint32_t order, uint64_t n_lanes, const void *t, uint64_t n_rows,
+                                        void *out, void *stream);
 extern "C" int hyk_generic_fp64_peak(int device, double millis, double *flops_per_s, char *err, size_t errlen);
 extern "C" int hyk_generic_fp32_peak(int device, double millis, double *flops_per_s, char *err, size_t errlen);
 extern "C" int hyk_generic_count_finished(const uint32_t *status, uint64_t n_lanes, uint32_t *finished, void *stream);
@@ -1237,6 +1240,15 @@ int hyk_dense_eval(const double *tc, uint32_t n_eq, uint32_t order, uint64_t n_l
     return 0;
 }
 
+int hyk_coutput_eval(int f32, const void *tcs, const void *t_hi, const void *t_lo, uint64_t n_steps, uint32_t n_eq,
+                     uint32_t order, uint64_t n_lanes, const void *t, uint64_t n_rows, void *out, void *stream) {
+    if (n_lanes == 0 || n_rows == 0) return 0;
+    if (!tcs || !t_hi || !t_lo || !t || !out || n_steps == 0 || n_eq == 0)
+        return fail(HYK_ERR_INVALID, "invalid continuous-output arguments");
+    const int rc = hyk_generic_coutput_eval(f32, tcs, t_hi, t_lo, n_steps, n_eq, order, n_lanes, t, n_rows, out, stream);
+    if (rc) return fail(HYK_ERR_CUDA, "continuous-output kernel launch failed");
+    return 0;
+}
 int hyk_dense_eval_f32(const float *tc, uint32_t n_eq, uint32_t order, uint64_t n_lanes, uint64_t ld, const float *dt,
                        float *out, void *stream) {
     if (n_lanes == 0) return 0;

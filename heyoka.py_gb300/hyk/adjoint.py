@@ -33,11 +33,19 @@ EPS = 2.220446049250313e-16
 LONGEST_FIRST = True
 
 
-def _propagate_taped(mod, x, pars, t0, tf, cap=64):
+def _tape_cap(ne, B):
+    # Steps per lane of a new tape: what 512 MiB hold, 64 at least and 1024 at
+    # most.  A lane that fills it stops, and is resumed by another launch after
+    # the tape has been copied to a larger one.
+    return min(1024, max(64, (1 << 29) // ((ne + 2) * 8 * max(B, 1))))
+
+
+def _propagate_taped(mod, x, pars, t0, tf, cap=None):
     """Propagate lanes (x: (n_eq, B)) from t0 to tf (B,), taping every step."""
     L = _lib.load()
     dev = x.device
     ne, B = x.shape
+    cap = _tape_cap(ne, B) if cap is None else cap
     f64 = dict(dtype=torch.float64, device=dev)
     th = t0.clone().contiguous()
     tl = torch.zeros(B, **f64)

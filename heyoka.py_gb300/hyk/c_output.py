@@ -12,7 +12,7 @@ Evaluation runs on the GPU: for each lane the step containing t is found by a
 batched binary search over the lane's end times (the last step whose start
 time is <= t, clamped to the first/last step outside the range), and the
 state polynomial is evaluated by Horner at the double-length offset from the
-step start (libhyk's dense-output kernel).
+step start (libhyk's hyk_coutput_eval, one launch for all the times).
 """
 
 from __future__ import annotations
@@ -25,19 +25,6 @@ import torch
 from . import _lib
 from .core import stream_handle
 from .integrator import _owned
-
-
-def _two_sum(a, b):
-    s = a + b
-    bb = s - a
-    return s, (a - (s - bb)) + (b - bb)
-
-
-def _dsub_hi(ah, bh, bl):
-    # hi part of (ah, 0) - (bh, bl) in double-length arithmetic
-    s, e = _two_sum(ah, -bh)
-    e = e + (0.0 - bl)
-    return s + e
 
 
 _DEFAULT_MSG = "Cannot use a default-constructed continuous_output_batch object"
@@ -69,12 +56,6 @@ class continuous_output_batch:
         self._dim = tcs.shape[1]
         self._out = None
         self._nit = n_iter
-        n = self._tcs.shape[0]
-        if n:
-            # Search keys: start times of the steps, sign-normalised per lane
-            # so that they are non-decreasing for backward propagations too.
-            self._sgn = torch.where(self._thi[-1] < self._thi[0], -1.0, 1.0).to(tcs.dtype)
-            self._keys = (self._thi[:n] * self._sgn).t().contiguous()  # (B, n)
 
     def _check(self):
         if self._tcs is None:
@@ -117,23 +98,17 @@ class continuous_output_batch:
         t = self._thi.cpu().numpy()
         return (np.array(t[0]), np.array(t[-1]))
 
-    def _eval_row(self, t):
-        n = self.n_steps
-        idx = torch.searchsorted(self._keys, (t * self._sgn).view(self._B, 1).contiguous(), right=True).view(self._B)
-        idx = (idx - 1).clamp(0, n - 1)
-        lanes = torch.arange(self._B, device=self._dev)
-        tc = self._tcs[idx, :, :, lanes].permute(1, 2, 0).contiguous()  # (dim, order+1, B)
-        dt = _dsub_hi(t, self._thi[idx, lanes], self._tlo[idx, lanes]).contiguous()
-        out = torch.empty((self._dim, self._B), dtype=self._tcs.dtype, device=self._dev)
-        L = _lib.load()
-        fn = L.hyk_dense_eval_f32 if self._tcs.dtype == torch.float32 else L.hyk_dense_eval
+    def _eval_rows(self, t):
+        """The states at the times t ((n, batch_size), contiguous, on the device)."""
+        out = torch.empty((t.shape[0], self._dim, self._B), dtype=self._tcs.dtype, device=self._dev)
         with torch.cuda.device(self._dev):
             _lib.check(
-                fn(
-                    tc.data_ptr(), self._dim, self._order, self._B, self._B, dt.data_ptr(), out.data_ptr(),
-                    stream_handle(self._dev.index),
+                _lib.load().hyk_coutput_eval(
+                    int(self._tcs.dtype == torch.float32), self._tcs.data_ptr(), self._thi.data_ptr(),
+                    self._tlo.data_ptr(), self.n_steps, self._dim, self._order, self._B, t.data_ptr(), t.shape[0],
+                    out.data_ptr(), stream_handle(self._dev.index),
                 ),
-                "hyk_dense_eval",
+                "hyk_coutput_eval",
             )
         return out
 
@@ -165,17 +140,16 @@ class continuous_output_batch:
                     "Invalid time array passed to a continuous_output_batch object: the length must be {} "
                     "but it is {} instead".format(self._B, t.shape[0])
                 )
-            self._out = self._eval_row(t)
+            self._out = self._eval_rows(t.reshape(1, -1).contiguous())[0]
             return self.output
         if t.shape[1] != self._B:
             raise ValueError(
                 "Invalid time array passed to a continuous_output_batch object: the number of columns must be "
                 "{} but it is {} instead".format(self._B, t.shape[1])
             )
-        rows = [self._eval_row(t[i].contiguous()) for i in range(t.shape[0])]
-        if rows:
-            self._out = rows[-1]
-        res = torch.stack(rows) if rows else torch.empty((0, self._dim, self._B), dtype=dt)
+        res = self._eval_rows(t.contiguous())
+        if t.shape[0]:
+            self._out = res[-1].clone()
         return _owned(res.cpu().numpy(), self)
 
     def lanes(self, sl):

@@ -1022,7 +1022,10 @@ class taylor_adaptive_batch:
         cap = 0
         tcs = thi = tlo = None
         if c_output:
-            cap = 64
+            # room for as many steps as 512 MiB hold (64 at least, 1024 at most):
+            # a lane that fills it stops and is resumed by another launch
+            # after the records have been copied to a larger store
+            cap = min(1024, max(64, (1 << 29) // (ne * (order + 1) * B * self._state.element_size())))
             tcs = torch.empty((cap, ne, order + 1, B), dtype=self._tdt, device=self._tdev)
             thi = torch.empty((cap, B), dtype=self._tdt, device=self._tdev)
             tlo = torch.empty((cap, B), dtype=self._tdt, device=self._tdev)
@@ -1224,12 +1227,11 @@ class taylor_adaptive_batch:
         K = int(nit.max().item()) if B else 0
         ne, order = self.dim, self._order
         fr = dict(dtype=self._tdt, device=self._tdev)
-        out_tcs = torch.empty((K, ne, order + 1, B), **fr)
+        out_tcs = torch.empty((0, ne, order + 1, B), **fr)
         out_thi = torch.empty((K + 1, B), **fr)
         out_tlo = torch.empty((K + 1, B), **fr)
         out_thi[0], out_tlo[0] = t0h, t0l
         if K:
-            out_tcs.copy_(tcs[:K])
             out_thi[1:].copy_(thi[:K])
             out_tlo[1:].copy_(tlo[:K])
             # Zero steps of lanes that finished early: final-state jets, final time.
@@ -1237,7 +1239,7 @@ class taylor_adaptive_batch:
             self._refresh_final_tc()
             idx = torch.arange(K, device=self._tdev).view(K, 1)
             pad = idx >= nit.view(1, B)
-            out_tcs = torch.where(pad.view(K, 1, 1, B), self._tc.unsqueeze(0), out_tcs)
+            out_tcs = torch.where(pad.view(K, 1, 1, B), self._tc.unsqueeze(0), tcs[:K])
             out_thi[1:] = torch.where(pad, self._thi.view(1, B), out_thi[1:])
             out_tlo[1:] = torch.where(pad, self._tlo.view(1, B), out_tlo[1:])
         return continuous_output_batch(out_tcs, out_thi, out_tlo, order, nit.clone())

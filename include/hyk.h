@@ -452,6 +452,14 @@ int hyk_adjoint(hyk_module *m, const hyk_lanes_t *lanes, const double *ck_x, con
 int hyk_dense_eval(const double *tc, uint32_t n_eq, uint32_t order, uint64_t n_lanes, uint64_t ld,
                    const double *dt, double *out, void *stream);
 
+/* Continuous output (heyoka/taylor_expose_c_output.cpp:272-408) at n_rows times
+ * per lane: tcs (n_steps, n_eq, order + 1, n_lanes), t_hi and t_lo
+ * (n_steps + 1, n_lanes) the steps' start times (the last row the end), t
+ * (n_rows, n_lanes), out (n_rows, n_eq, n_lanes); double, or float when f32.  A
+ * time outside the lane's steps is evaluated on the first or last of them. */
+int hyk_coutput_eval(int f32, const void *tcs, const void *t_hi, const void *t_lo, uint64_t n_steps, uint32_t n_eq,
+                     uint32_t order, uint64_t n_lanes, const void *t, uint64_t n_rows, void *out, void *stream);
+
 /* Dense output of a single-precision module (float arrays, the same layout). */
 int hyk_dense_eval_f32(const float *tc, uint32_t n_eq, uint32_t order, uint64_t n_lanes, uint64_t ld,
                        const float *dt, float *out, void *stream);
