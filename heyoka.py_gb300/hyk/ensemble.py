@@ -54,15 +54,26 @@ def _host_copy(ta):
     return new
 
 
-def _clone_host(tmpl):
-    # A fresh host copy from the host template: CPU tensor clones only (the
-    # device is read once per ensemble, not once per iteration).  Events are
+def _host_rows(tmpl, n_iter):
+    # The tensors of every iteration's host copy, as rows of one stacked tensor
+    # per name: {name: (stacked, its rows)}.
+    rows = {}
+    for k, v in tmpl.__dict__.items():
+        if isinstance(v, torch.Tensor):
+            stacked = v.unsqueeze(0).repeat(n_iter, *([1] * v.dim()))
+            rows[k] = (stacked, stacked.unbind(0))
+    return rows
+
+
+def _clone_host(tmpl, rows, i):
+    # Iteration i's host copy of the host template: its own rows of CPU tensors
+    # (the device is read once per ensemble, not once per iteration).  Events are
     # deep-copied, as the reference's per-iteration deep copy does, so every
     # iteration has its own callback objects.
     new = object.__new__(type(tmpl))
     for k, v in tmpl.__dict__.items():
-        if isinstance(v, torch.Tensor):
-            new.__dict__[k] = v.clone()
+        if k in rows:
+            new.__dict__[k] = rows[k][1][i]
         elif k in ("_t_events", "_nt_events"):
             new.__dict__[k] = _copy.deepcopy(v)
         elif k == "_ev":
@@ -188,15 +199,16 @@ def _ensemble(tp, ta, arg, n_iter, gen, **kwargs):
         return []
     B = ta.batch_size
     tmpl = _host_copy(ta)
+    rows = _host_rows(tmpl, n_iter)
     scopies = None
     if scalar:
-        scopies = [gen(taylor_adaptive._wrap(_clone_host(tmpl)), i) for i in range(n_iter)]
+        scopies = [gen(taylor_adaptive._wrap(_clone_host(tmpl, rows, i)), i) for i in range(n_iter)]
         for sc in scopies:
             if not isinstance(sc, taylor_adaptive):
                 raise TypeError("the ensemble generator must return the integrator it was given")
         copies = [sc._b for sc in scopies]
     else:
-        copies = [gen(_clone_host(tmpl), i) for i in range(n_iter)]
+        copies = [gen(_clone_host(tmpl, rows, i), i) for i in range(n_iter)]
     for c in copies:
         if not isinstance(c, taylor_adaptive_batch) or c.batch_size != B or c._dec is not ta._dec:
             raise TypeError("the ensemble generator must return the integrator it was given")
@@ -207,7 +219,18 @@ def _ensemble(tp, ta, arg, n_iter, gen, **kwargs):
     big._B = n_iter * B
     # the kernel form for the whole ensemble, not for one iteration's batch
     big._mod = ta._module_for(big._B)
-    cat = lambda name: torch.cat([getattr(c, name).cpu() for c in copies], dim=-1).to(dev).contiguous()  # noqa: E731
+
+    def cat(name):
+        # (lanes last) the stacked rows in one transfer, or, where a generator
+        # put another tensor in a row's place or returned its copies in another
+        # order, the copies' tensors one by one
+        stacked, own = rows[name]
+        if all(getattr(c, name) is r for c, r in zip(copies, own)):
+            v = stacked.to(dev)
+            k = v.dim() - 2
+            return v.permute(*range(1, k + 1), 0, k + 1).reshape(*v.shape[1:-1], n_iter * B).contiguous()
+        return torch.cat([getattr(c, name).cpu() for c in copies], dim=-1).to(dev).contiguous()
+
     big._state = cat("_state")
     big._pars = cat("_pars")
     big._thi = cat("_thi")
@@ -272,8 +295,9 @@ def _ensemble(tp, ta, arg, n_iter, gen, **kwargs):
         res = big._run(tf_hi, tf_lo, ms, md, write_tc=bool(kwargs.get("write_tc", False)),
                        c_output=bool(kwargs.get("c_output", False)), group=B, group_callbacks=gcb)
     big._refresh_final_tc()
-    parts = {name: _split(getattr(big, name), n_iter, B) for name in ("_state", "_pars", "_thi", "_tlo", "_last_h", "_tc", "_d_out")}
-    prop = {k: (None if v is None else _split(v, n_iter, B)) for k, v in big._prop.items()}
+    parts = {name: _split(getattr(big, name), n_iter, B).unbind(0)
+             for name in ("_state", "_pars", "_thi", "_tlo", "_last_h", "_tc", "_d_out")}
+    prop = {k: (None if v is None else _split(v, n_iter, B).unbind(0)) for k, v in big._prop.items()}
     grid_np = None
     if tp == "grid":
         g = res["grid_out"].cpu().numpy()

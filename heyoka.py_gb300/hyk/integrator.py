@@ -208,7 +208,8 @@ class LaneArray(torch.Tensor):
         return torch.as_tensor(a, device=self.device)
 
     def __setitem__(self, idx, value):
-        super().__setitem__(idx, self._coerce(value))
+        # on the plain tensor: the subclass's dispatch costs more than the copy
+        self.as_subclass(torch.Tensor)[idx] = self._coerce(value)
 
     # Comparisons give host NumPy arrays, as comparisons of the reference's views do.
     def __eq__(self, other):
@@ -791,8 +792,10 @@ class taylor_adaptive_batch:
         return torch.tensor(a, dtype=self._tdt, device=self._tdev)
 
     def set_time(self, time):
-        t = self._lane_vec(time, "time vector")
-        self._thi.copy_(t)
+        if _is_scalar(time):
+            self._thi.fill_(float(self._np_dt(time)))
+        else:
+            self._thi.copy_(self._lane_vec(time, "time vector"))
         self._tlo.zero_()
 
     def set_dtime(self, hi_time, lo_time):
@@ -833,7 +836,7 @@ class taylor_adaptive_batch:
                 "hyk_step",
             )
         self._step_res = (oc, h)
-        self._last_h = h.clone()
+        self._last_h = h
         if write_tc:
             self._final_tc_mask = None
         if self._ev is not None:
@@ -935,6 +938,11 @@ class taylor_adaptive_batch:
         }
         return p
 
+    def _ev_t_callbacks(self):
+        """Whether a terminal event may have a callback (of an ensemble's
+        iterations, whose events are copies of these)."""
+        return "_ev_route" in self.__dict__ or any(e.callback is not None for e in self._t_events)
+
     def _ev_has_callbacks(self):
         return bool(self._nt_events) or any(e.callback is not None for e in self._t_events)
 
@@ -972,7 +980,7 @@ class taylor_adaptive_batch:
                 None if self._ev is None else {k: self._ev[k].clone() for k in ("count", "last", "sign")})
         res = self._run_once(tf_hi, tf_lo, max_steps, md, grid, write_tc, c_output, group, lane_order, callback,
                              group_callbacks, (stop, G), False)
-        if bool((stop != -1).any()):
+        if bool(((stop.cpu() if stop.numel() <= 4096 else stop) != -1).any()):
             # a state became non-finite: run again from the initial state, every
             # lane of the group taking the failing iteration uncounted and stopping
             self._state.copy_(snap[0])
@@ -1029,7 +1037,9 @@ class taylor_adaptive_batch:
             tcs = torch.empty((cap, ne, order + 1, B), dtype=self._tdt, device=self._tdev)
             thi = torch.empty((cap, B), dtype=self._tdt, device=self._tdev)
             tlo = torch.empty((cap, B), dtype=self._tdt, device=self._tdev)
-        t0h, t0l = self._thi.clone(), self._tlo.clone()
+        # whether lanes queue behind the first round, whose order then matters
+        queued = self._schedule == "lpt" and B >= 4096 and B > self._first_round(grid is not None)
+        t0h, t0l = (self._thi.clone(), self._tlo.clone()) if (c_output or queued) else (None, None)
 
         def desc():
             return self._ev_fill(_lib.hyk_prop_t(
@@ -1051,7 +1061,7 @@ class taylor_adaptive_batch:
 
         lanes = lanes_struct(self._state, self._pars, self._thi, self._tlo)
         mode = _lib.HYK_MODE_PERSISTENT if (self._prop_mode == "persistent" or stepped) else _lib.HYK_MODE_PLAIN
-        if lane_order is None and mode == _lib.HYK_MODE_PERSISTENT and self._schedule == "lpt" and B >= 4096:
+        if lane_order is None and mode == _lib.HYK_MODE_PERSISTENT and queued:
             lane_order = self._lpt_order(tf_hi, tf_lo)
         done_mask = _lib.LANE_DONE | _lib.LANE_STOPPED
         g_open = None
@@ -1107,7 +1117,7 @@ class taylor_adaptive_batch:
                 if self._ev is not None:
                     self._ev_dispatch_nt()
                     evl = (p["status"] & _lib.LANE_EVENT) != 0
-                    if bool(evl.any()):
+                    if self._ev_t_callbacks() and bool(evl.any()):
                         idx = torch.nonzero(evl).flatten().cpu().numpy()
                         ks = p["outcome"][evl].cpu().numpy()
                         resume = self._ev_terminal({int(b): -int(k) - 1 for b, k in zip(idx, ks)})
@@ -1161,8 +1171,9 @@ class taylor_adaptive_batch:
         # Each lane's steps per unit of time over this propagation: the next
         # longest-first queue's estimate of its work (orbits whose step size
         # varies along the orbit are poorly predicted by one step size).
-        span = ((self._thi.double() - t0h.double()) + (self._tlo.double() - t0l.double())).abs()
-        self._step_rate = torch.where(span > 0, p["n_steps"].double() / span, torch.zeros_like(span))
+        if queued:
+            span = ((self._thi.double() - t0h.double()) + (self._tlo.double() - t0l.double())).abs()
+            self._step_rate = torch.where(span > 0, p["n_steps"].double() / span, torch.zeros_like(span))
         res = {"grid_out": grid_out}
         if c_output:
             nrec = p["n_iter"]
@@ -1174,33 +1185,45 @@ class taylor_adaptive_batch:
             res["c_output"] = self._make_c_output(p, tcs, thi, tlo, t0h, t0l, nrec)
         return res
 
+    def _first_round(self, with_grid):
+        """How many trajectories start at once, one warp per SM sub-partition
+        (or, in the team form, on every resident warp): up to this size no lane
+        waits for another, and the order of the queue does not matter."""
+        mod = self._mod_grid if (with_grid and self.__dict__.get("_mod_grid") is not None) else self._mod
+        i = mod.info
+        warps = i.ctas_per_sm * (i.block_lanes // 32)
+        return i.n_sm * (warps if i.team_size > 1 else min(warps, 4)) * (32 // i.team_size)
+
     def _lpt_order(self, tf_hi, tf_lo):
         """Longest-first queue order for the persistent kernel: lanes sorted by
         the estimated number of steps, the lane's measured steps per unit of
-        time over its previous propagation times |t_final - t|, or, for a lane
-        without one, |t_final - t| / h, h the size of a step from the current
+        time over its previous propagation times |t_final - t| (lanes that
+        did not move in it first), or, without a previous propagation,
+        |t_final - t| / h, h the size of a step from the current
         state (one extra step evaluation, not applied).  The order changes
         only the schedule, never a lane's arithmetic."""
-        L = _lib.load()
         B = self._B
-        st, th, tl = self._state.clone(), self._thi.clone(), self._tlo.clone()
-        oc = torch.empty(B, dtype=torch.int64, device=self._tdev)
-        h = torch.empty(B, dtype=self._tdt, device=self._tdev)
-        with torch.cuda.device(self._dev):
-            _lib.check(
-                L.hyk_step(self._mod.handle, lanes_struct(st, self._pars, th, tl), None, 0, oc.data_ptr(),
-                           h.data_ptr(), None, self._ev_scratch(), stream_handle(self._dev)),
-                "hyk_step",
-            )
         rem = (tf_hi.double() - self._thi.double()).abs()
         if tf_lo is not None:
             rem = (rem + tf_lo.double().abs())
-        est = torch.nan_to_num(rem / h.double().abs(), nan=0.0, posinf=1e300)
         rate = self.__dict__.get("_step_rate")
-        if rate is not None and rate.numel() == B and rate.device == est.device:
-            # lanes with a previous propagation: its measured step rate
-            est = torch.where(rate > 0, rate * rem, est)
-        return torch.argsort(est, descending=True).contiguous()
+        if rate is not None and rate.numel() == B and rate.device == rem.device:
+            # lanes with a previous propagation: its measured step rate (the
+            # others first)
+            est = torch.where(rate > 0, rate * rem, math.inf)
+        else:
+            L = _lib.load()
+            st, th, tl = self._state.clone(), self._thi.clone(), self._tlo.clone()
+            oc = torch.empty(B, dtype=torch.int64, device=self._tdev)
+            h = torch.empty(B, dtype=self._tdt, device=self._tdev)
+            with torch.cuda.device(self._dev):
+                _lib.check(
+                    L.hyk_step(self._mod.handle, lanes_struct(st, self._pars, th, tl), None, 0, oc.data_ptr(),
+                               h.data_ptr(), None, self._ev_scratch(), stream_handle(self._dev)),
+                    "hyk_step",
+                )
+            est = torch.nan_to_num(rem / h.double().abs(), nan=0.0, posinf=1e300)
+        return torch.argsort(est.float(), descending=True).contiguous()
 
     def _finish_prop(self, p, group, last_tc):
         """Apply the whole-batch rules that couple the lanes of a batch."""
@@ -1246,7 +1269,9 @@ class taylor_adaptive_batch:
 
     def _check_time(self, t, what):
         tt = self._lane_vec(t, what)
-        if not bool(torch.isfinite(tt).all()):
+        # (a scalar is looked at on the host: no launch, no wait)
+        ok = math.isfinite(float(self._np_dt(t))) if _is_scalar(t) else bool(torch.isfinite(tt).all())
+        if not ok:
             raise ValueError(
                 "A non-finite time was passed to the propagate_until() function of an adaptive Taylor integrator"
             )
