@@ -335,49 +335,52 @@ static uint32_t default_team(const hyk::TeamInfo &ti, size_t lane_bytes, size_t 
 //
 // A team of T threads issues 1 / (T util) of them; a warp alone on its
 // sub-partition takes c times its FP64 time (1.15 measured for the lane form,
-// 1.8 for teams, whose operands come through descriptors), and k warps on one
-// (c^4 + k^4)^(1/4).  A small batch cannot fill the warps of the lane form,
-// so a team that spreads each trajectory wins there: 331 six-body members
-// take 76 us a step with teams of 32 and 99 with 16, 3001 of them 287 and 214
-// (estimated 0.095, 0.127, 0.264, 0.197); 1003 Kepler orbits 58 us in the lane
-// form and 53 with teams of 8.  Lane-form systems so large that their
-// recurrences are split into functions and still spill are counted at c = 4
-// (first-order variational Kepler, 42 equations: 2.05 ms a step in the lane
-// form, 139 us with teams of 32; ptxas 41 s and 0.8 s).  The default form
-// is kept unless another is estimated 5 % faster, and of the teams above the
-// fastest the first within 12 % of it is taken: trajectories of one batch end
-// at different times, and the last ones then run fastest (3001 variational
-// Kepler orbits to t = 10: 47.6 ms with teams of 8, 42.1 with 16).
-// Whole calls, lane form and the choice: 3001 variational Kepler orbits 463 and
-// 42 ms, 331 six-body members (teams of 16 before) 8.1 and 5.0 ms, 1003 Kepler
-// orbits 51.7 and 48.7 ms.
+// 1.55 for teams), and w warps on one (c^4 + w^4)^(1/4), w at most what is
+// resident.  Trajectories of one batch end at different times, so that the warps
+// at work are counted at 0.7 of those at the start.  A small batch cannot fill
+// the warps of the lane form, so a team that spreads each trajectory wins
+// there.  Measured, us a step (estimated, in lane-form steps): 331 six-body
+// members with teams of 32 and 16 69 and 100 (0.082, 0.109), 3001 of them 249 and
+// 185 (0.185, 0.138); Kepler in the lane form and with teams of 4 59 and 47 for
+// 1003 orbits (1.15, 0.88), 59 and 53 for 10007 (1.15, 1.02), 59 and 83 for 20011
+// (1.15, 1.67).  Lane-form systems so large that their recurrences are split into
+// functions and still spill are counted at c = 4 (first-order variational Kepler,
+// 42 equations: 2.05 ms a step in the lane form, 127 us with teams of 32; ptxas
+// 41 s and 0.8 s).  The default form is kept unless another is estimated 5 %
+// faster, and of teams within 12 % of the fastest the one with the fewest
+// instructions is taken, the smallest if several have as few: the last
+// trajectories then run fastest (3001 variational Kepler orbits with teams of 8
+// and 16 12.6 and 11.8 ms; 1003 Kepler orbits with 4 and 16 3.49 and 3.73 ms).
 static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool large, size_t real_bytes, const Device &dv,
                                uint64_t n) {
     const double smsp = 4.0 * dv.n_sm;
     auto cost = [&](double c, double warps, double resident) {
-        const double w = std::ceil(warps / smsp - 1e-9), k = std::max(1.0, std::min(resident, w));
+        const double w = 0.7 * warps / smsp, k = std::min(resident, w);
         const double t = w <= 1.0 ? c : std::pow(c * c * c * c + k * k * k * k, 0.25);
-        return t * std::max(1.0, warps / smsp / k);
+        return t * std::max(1.0, w / std::max(k, 1.0));
     };
-    double c[6];
+    double c[6], instr[6];
     c[0] = cost(large ? 4.0 : 1.15, (double)n / 32.0, 2.0);
+    instr[0] = 1.0;
     for (uint32_t l = 1; l <= 5; ++l) {
         const uint32_t T = 1u << l;
         const uint32_t slots = ti.n_slot_cold ? ti.n_slot_cold : ti.n_slot;
         const size_t cta = (size_t)(32 / T) * slots * real_bytes;
         c[l] = INFINITY;
+        instr[l] = 1.0 / (T * ti.util[l]);
         if (cta > (size_t)dv.smem_optin) continue;
-        const double resident = std::min(24.0, (double)((size_t)dv.smem_per_sm / (cta + 1024))) / 4.0;
-        c[l] = cost(1.8, (double)n * T / 32.0, resident) / (T * ti.util[l]);
+        const double resident = std::min(16.0, (double)((size_t)dv.smem_per_sm / (cta + 1024))) / 4.0;
+        c[l] = cost(1.55, (double)n * T / 32.0, resident) * instr[l];
     }
     const uint32_t dl = dflt ? (uint32_t)__builtin_ctz(dflt) : 0;
     uint32_t best = 0;
     for (uint32_t l = 1; l <= 5; ++l)
-        if (c[l] <= c[best]) best = l;
-    if (c[best] * 1.05 >= c[dl]) return dflt;
-    for (uint32_t l = best + 1; best && l <= 5; ++l)
-        if (c[l] <= 1.12 * c[best]) return 1u << l;
-    return best ? 1u << best : 0;
+        if (c[l] < c[best]) best = l;
+    if (best == 0 || c[best] * 1.05 >= c[dl]) return c[best] * 1.05 < c[dl] ? 0 : dflt;
+    uint32_t pick = best;
+    for (uint32_t l = 1; l <= 5; ++l)
+        if (c[l] <= 1.12 * c[best] && instr[l] < 0.98 * instr[pick]) pick = l;
+    return 1u << pick;
 }
 
 extern "C" {
