@@ -291,7 +291,7 @@ struct Gen {
     // other such operations) are constant in time: only their order-0 value
     // exists (one slot, like a parameter) and their higher orders are known
     // zeros, so products with them are single terms.  Gpu arithmetic only;
-    // the pinned arithmetic and the adjoint keep the full recurrences.
+    // the pinned arithmetic keeps the full recurrences.
     std::vector<char> cst;
 
     // Cold state rows (coldrows mode): a state variable whose coefficients no
@@ -361,7 +361,7 @@ struct Gen {
                 base[u] = base[op.a.idx];
                 negf[u] = !negf[op.a.idx];
             }
-            if (!pin && !adj) {
+            if (!pin) {
                 auto kconst = [&](const hyk_arg_t &a) {
                     return a.kind == HYK_ARG_NONE || a.kind == HYK_ARG_NUM || a.kind == HYK_ARG_PAR ||
                            (a.kind == HYK_ARG_U && cst[base[a.idx]]);
@@ -555,7 +555,7 @@ struct Gen {
             for (uint32_t k = 0; k < d.n_ops; ++k) {
                 const uint32_t u = N + k;
                 const int o = d.ops[k].op;
-                if (alias[u] || p < 2 || ((o == HYK_OP_ADD || o == HYK_OP_SUB || o == HYK_OP_NEG) && !fused_sq(u)))
+                if (alias[u] || cst[u] || p < 2 || ((o == HYK_OP_ADD || o == HYK_OP_SUB || o == HYK_OP_NEG) && !fused_sq(u)))
                     continue;
                 aslot[u] = (int)s;
                 s += p - 1;
@@ -1129,10 +1129,20 @@ struct Gen {
     // ub(r) += e (r a variable, or a parameter at order 0).
     // (as fused multiply-adds, which the FP64 pipe issues fastest; scale:
     // ub(r) += scale * e).
+    // The first contribution to an operation's adjoint sets it (0 + e = e).
+    std::vector<char> ubset;
     void contrib(const Ref &r, uint32_t m, const std::string &e, const std::string &scale = "") {
         std::string f = scale.empty() ? "hyk_one" : scale;
         if (r.neg) f = "(-" + f + ")";
-        if (r.kind == HYK_ARG_U) {
+        if (r.kind == HYK_ARG_U && !ubset[r.u]) {
+            ubset[r.u] = 1;
+            const bool one = f == "hyk_one" || f == "(-(-hyk_one))", minus = f == "(-hyk_one)";
+            o << "    " << ub((uint32_t)r.u) << " = ";
+            if (one || minus)
+                o << (minus ? "-(" : "") << e << (minus ? ")" : "") << ";\n";
+            else
+                o << "__fma_rn(" << f << ", " << e << ", hyk_nz);\n";
+        } else if (r.kind == HYK_ARG_U) {
             o << "    " << ub((uint32_t)r.u) << " = __fma_rn(" << f << ", " << e << ", " << ub((uint32_t)r.u) << ");\n";
         } else if (r.kind == HYK_ARG_PAR && m == 0) {
             o << "    pb[" << r.par << "] = __fma_rn(" << f << ", " << e << ", pb[" << r.par << "]);\n";
@@ -1162,6 +1172,8 @@ struct Gen {
         if (alias[u]) return;
         const Ref A = res(op.a), B = res(op.b);
         const Ref self{HYK_ARG_U, (int)u, false, 0, -1};
+        if (cst[u] && m >= 1) return;  // constant in time: its order 0 only
+        const uint32_t lim = cst[u] ? m + 1 : p;  // the orders it has
         const bool unary_fn = op.op == HYK_OP_SQRT || op.op == HYK_OP_POW || op.op == HYK_OP_EXP ||
                               op.op == HYK_OP_LOG || op.op == HYK_OP_SIN || op.op == HYK_OP_COS;
         // A function of a constant is constant: nothing flows back above order 0.
@@ -1172,8 +1184,9 @@ struct Gen {
             // c_n = a_n + sum_i k_i t_i,n: abar_m += cbar_m, tbar_i,m += k_i cbar_m
             const Ref FA = fz_a(u);
             const std::vector<Ref> FX = fz_x(u);
-            if (FA.kind == HYK_ARG_U) contrib(FA, m, G);
-            for (size_t i = 0; i < FX.size(); ++i) contrib(FX[i], m, G, lit(fz_k(u)[i]));
+            if (FA.kind == HYK_ARG_U && nz(FA, m)) contrib(FA, m, G);
+            for (size_t i = 0; i < FX.size(); ++i)
+                if (nz(FX[i], m)) contrib(FX[i], m, G, lit(fz_k(u)[i]));
             return;
         }
         if (fused(u)) {
@@ -1182,11 +1195,12 @@ struct Gen {
             const Ref FA = fz_a(u);
             o << "    const double " << H << " = " << G << ";\n";
             keep(u, m);
-            if (FA.kind == HYK_ARG_U) contrib(FA, m, H);
+            if (FA.kind == HYK_ARG_U && nz(FA, m)) contrib(FA, m, H);
             for (const Ref &x : fz_x(u)) {
                 t.clear();
-                if (wants(x, m))
-                    for (uint32_t n = m; n < p; ++n) t.push_back({hval(u, n, m), val(x, n - m)});
+                if (nz(x, m) && wants(x, m))
+                    for (uint32_t n = m; n < lim; ++n)
+                        if (nz(x, n - m)) t.push_back({hval(u, n, m), val(x, n - m)});
                 const std::string sx = gsum(t);
                 if (!sx.empty()) contrib(x, m, sx, "2.0");
             }
@@ -1209,13 +1223,13 @@ struct Gen {
             o << "    const double " << H << " = " << G << ";\n";
             keep(u, m);
             if (nz(A, m) && wants(A, m))
-                for (uint32_t n = m; n < p; ++n)
+                for (uint32_t n = m; n < lim; ++n)
                     if (nz(B, n - m)) t.push_back({hval(u, n, m), val(B, n - m)});
             const std::string sa = gsum(t);
             if (!sa.empty()) contrib(A, m, sa);
             t.clear();
             if (nz(B, m) && wants(B, m))
-                for (uint32_t n = m; n < p; ++n)
+                for (uint32_t n = m; n < lim; ++n)
                     if (nz(A, n - m)) t.push_back({hval(u, n, m), val(A, n - m)});
             const std::string sb = gsum(t);
             if (!sb.empty()) contrib(B, m, sb);
@@ -1224,7 +1238,7 @@ struct Gen {
         case HYK_OP_DIV: {
             // c_n = (a_n - sum_{j>=1} b_j c_{n-j}) / b_0, w_n = cbar_n / b_0:
             // cbar_m -= sum_{n>m} w_n b_{n-m}; abar_m += w_m; bbar_m -= sum_{n>=m} w_n c_{n-m}.
-            for (uint32_t n = m + 1; n < p; ++n)
+            for (uint32_t n = m + 1; n < lim; ++n)
                 if (nz(B, n - m)) t.push_back({hval(u, n, m), val(B, n - m)});
             const std::string ss = gsum(t);
             if (!ss.empty()) o << "    " << G << " = " << G << " - " << ss << ";\n";
@@ -1233,7 +1247,7 @@ struct Gen {
             if (nz(A, m)) contrib(A, m, H);
             t.clear();
             if (nz(B, m) && wants(B, m))
-                for (uint32_t n = m; n < p; ++n) t.push_back({hval(u, n, m), val(self, n - m)});
+                for (uint32_t n = m; n < lim; ++n) t.push_back({hval(u, n, m), val(self, n - m)});
             const std::string sb = gsum(t);
             if (!sb.empty()) contrib(B, m, sb, "(-hyk_one)");
             break;
@@ -1242,7 +1256,7 @@ struct Gen {
             o << "    const double " << H << " = " << G << ";\n";
             keep(u, m);
             if (nz(A, m) && wants(A, m))
-                for (uint32_t n = m; n < p; ++n)
+                for (uint32_t n = m; n < lim; ++n)
                     if (nz(A, n - m)) t.push_back({hval(u, n, m), val(A, n - m)});
             const std::string sa = gsum(t);
             if (!sa.empty()) contrib(A, m, sa, "2.0");
@@ -1251,7 +1265,7 @@ struct Gen {
         case HYK_OP_SQRT: {
             // c_n = (a_n - sum_{0<j<n} c_j c_{n-j}) / (2 c_0), w_n = cbar_n / (2 c_0):
             // cbar_m -= 2 sum_{n>m} w_n c_{n-m}; abar_m += w_m.
-            for (uint32_t n = m + 1; n < p; ++n) t.push_back({hval(u, n, m), val(self, n - m)});
+            for (uint32_t n = m + 1; n < lim; ++n) t.push_back({hval(u, n, m), val(self, n - m)});
             const std::string ss = gsum(t);
             if (!ss.empty()) o << "    " << G << " = __fma_rn(-2.0, " << ss << ", " << G << ");\n";
             o << "    const double " << H << " = __fma_rn(" << G << ", " << inv << ", hyk_nz);\n";
@@ -1265,7 +1279,7 @@ struct Gen {
             // abar_m += sum_{n>=m} w_n coef(n, n-m) c_{n-m} (m >= 1);
             // abar_0 += al cbar_0 c_0 / a_0 - sum_{n>=1} n w_n c_n.
             const double alpha = op.b.num;
-            for (uint32_t n = m + 1; n < p; ++n)
+            for (uint32_t n = m + 1; n < lim; ++n)
                 if (nz(A, n - m)) {
                     const double coef = (double)n * alpha - (double)m * (alpha + 1.0);
                     t.push_back({hval(u, n, m), "__fma_rn(" + lit(coef) + ", " + val(A, n - m) + ", hyk_nz)"});
@@ -1274,7 +1288,7 @@ struct Gen {
             if (!ss.empty()) o << "    " << G << " = " << G << " + " << ss << ";\n";
             t.clear();
             if (m == 0) {
-                for (uint32_t n = 1; n < p; ++n) t.push_back({hval(u, n, m), "__fma_rn(" + lit(-(double)n) + ", " + val(self, n) + ", hyk_nz)"});
+                for (uint32_t n = 1; n < lim; ++n) t.push_back({hval(u, n, m), "__fma_rn(" + lit(-(double)n) + ", " + val(self, n) + ", hyk_nz)"});
                 const std::string s0 = gsum(t);
                 std::string e = "(" + G + " * " + lit(alpha) + ") * (" + val(self, 0) + " * " + inv + ")";
                 if (!s0.empty()) e = "(" + e + " + " + s0 + ")";
@@ -1283,7 +1297,7 @@ struct Gen {
             }
             o << "    const double " << H << " = (" << G << " * " << inv << ") * " << lit(1.0 / (double)m) << ";\n";
             keep(u, m);
-            for (uint32_t n = m; n < p; ++n) {
+            for (uint32_t n = m; n < lim; ++n) {
                 const double coef = (double)n * alpha - (double)(n - m) * (alpha + 1.0);
                 t.push_back({hval(u, n, m), "__fma_rn(" + lit(coef) + ", " + val(self, n - m) + ", hyk_nz)"});
             }
@@ -1295,7 +1309,7 @@ struct Gen {
             // c_n = (1/n) sum_{j=1}^{n} (j a_j) c_{n-j}, w_n = cbar_n / n:
             // cbar_m += sum_{n>m} w_n (n-m) a_{n-m}; abar_m += m sum_{n>=m} w_n c_{n-m} (m >= 1);
             // abar_0 += cbar_0 c_0.
-            for (uint32_t n = m + 1; n < p; ++n)
+            for (uint32_t n = m + 1; n < lim; ++n)
                 if (knz(A, n - m)) t.push_back({hval(u, n, m), kval(A, n - m)});
             const std::string ss = gsum(t);
             if (!ss.empty()) o << "    " << G << " = " << G << " + " << ss << ";\n";
@@ -1307,7 +1321,7 @@ struct Gen {
             o << "    const double " << H << " = __fma_rn(" << G << ", " << lit(1.0 / (double)m) << ", hyk_nz);\n";
             keep(u, m);
             if (knz(A, m))
-                for (uint32_t n = m; n < p; ++n) t.push_back({hval(u, n, m), val(self, n - m)});
+                for (uint32_t n = m; n < lim; ++n) t.push_back({hval(u, n, m), val(self, n - m)});
             const std::string sa = gsum(t);
             if (!sa.empty()) contrib(A, m, sa, lit((double)m));
             break;
@@ -1318,13 +1332,13 @@ struct Gen {
             // abar_m += w_m - sum_{n>m} (w_n / n) (n-m) c_{n-m} (m >= 1);
             // abar_0 += cbar_0 / a_0 - sum_{n>=1} w_n c_n.
             if (m >= 1 && varying(A))
-                for (uint32_t n = m + 1; n < p; ++n)
+                for (uint32_t n = m + 1; n < lim; ++n)
                     if (nz(A, n - m)) t.push_back({hval(u, n, m), "__fma_rn(" + lit(1.0 / (double)n) + ", " + val(A, n - m) + ", hyk_nz)"});
             const std::string ss = gsum(t);
             if (!ss.empty()) o << "    " << G << " = __fma_rn(" << lit(-(double)m) << ", " << ss << ", " << G << ");\n";
             t.clear();
             if (m == 0) {
-                for (uint32_t n = 1; n < p; ++n) t.push_back({hval(u, n, m), val(self, n)});
+                for (uint32_t n = 1; n < lim; ++n) t.push_back({hval(u, n, m), val(self, n)});
                 const std::string s0 = gsum(t);
                 std::string e = "(" + G + " * " + inv + ")";
                 if (!s0.empty()) e = "(" + e + " - " + s0 + ")";
@@ -1335,7 +1349,7 @@ struct Gen {
             keep(u, m);
             std::string e = H;
             if (varying(A)) {
-                for (uint32_t n = m + 1; n < p; ++n)
+                for (uint32_t n = m + 1; n < lim; ++n)
                     t.push_back({hval(u, n, m), "__fma_rn(" + lit(1.0 / (double)n) + ", " + kval(self, n - m) + ", hyk_nz)"});
                 const std::string sa = gsum(t);
                 if (!sa.empty()) e = "(" + H + " - " + sa + ")";
@@ -1352,7 +1366,7 @@ struct Gen {
             const uint32_t partner = (uint32_t)op.aux;
             const bool is_sin = op.op == HYK_OP_SIN;
             const Ref P{HYK_ARG_U, (int)partner, false, 0, -1};
-            for (uint32_t n = m + 1; n < p; ++n)
+            for (uint32_t n = m + 1; n < lim; ++n)
                 if (knz(A, n - m)) t.push_back({hval(partner, n, m), kval(A, n - m)});
             const std::string ss = gsum(t);
             if (!ss.empty()) o << "    " << G << " = " << G << " + " << ss << ";\n";
@@ -1364,7 +1378,7 @@ struct Gen {
             o << "    const double " << H << " = __fma_rn(" << G << ", " << lit((is_sin ? 1.0 : -1.0) / (double)m) << ", hyk_nz);\n";
             keep(u, m);
             if (knz(A, m))
-                for (uint32_t n = m; n < p; ++n) t.push_back({hval(u, n, m), val(P, n - m)});
+                for (uint32_t n = m; n < lim; ++n) t.push_back({hval(u, n, m), val(P, n - m)});
             const std::string sa = gsum(t);
             if (!sa.empty()) contrib(A, m, sa, lit((double)m));
             break;
@@ -1374,17 +1388,11 @@ struct Gen {
         }
     }
 
-    void emit_inverses(bool only_used) {
-        (void)only_used;
+    // The order-0 reciprocals the forward recurrences kept (split functions).
+    void emit_inverses() {
         for (uint32_t k = 0; k < d.n_ops; ++k) {
-            const auto &op = d.ops[k];
             const uint32_t u = N + k;
-            if (alias[u]) continue;
-            const Ref A = res(op.a), B = res(op.b);
-            const std::string inv = "i" + std::to_string(u);
-            if (op.op == HYK_OP_DIV) o << "    const double " << inv << " = 1.0 / " << val(B, 0) << ";\n";
-            if (op.op == HYK_OP_POW || op.op == HYK_OP_LOG) o << "    const double " << inv << " = 1.0 / " << val(A, 0) << ";\n";
-            if (op.op == HYK_OP_SQRT) o << "    const double " << inv << " = 1.0 / (2.0 * sqrt(" << val(A, 0) << "));\n";
+            if (!alias[u] && islot[u] >= 0) o << "    const double " << inv0(u) << " = " << smem((uint32_t)islot[u]) << ";\n";
         }
     }
 
@@ -1397,12 +1405,12 @@ struct Gen {
         for (uint32_t m = 0; m < p; ++m) {
             gcount = 0;
             o << "static __device__ __noinline__ void hyk_bw_o" << m
-              << "(double *__restrict__ S, const double t0, const double h, double *__restrict__ lam, "
+              << "(double *__restrict__ S, const double t0, const double hm, double *__restrict__ lam, "
                  "double *__restrict__ pb) {\n";
+            ubset.assign(NU, 0);
+            for (uint32_t i = 0; i < N; ++i) ubset[i] = 1;
             o << "    (void)t0;\n    HYK_FMAOPS_CONSTS\n    (void)hyk_nz;\n";
-            emit_inverses(true);
-            o << "    double hm = 1.0;\n";
-            for (uint32_t q = 0; q < m; ++q) o << "    hm = hm * h;\n";
+            emit_inverses();
             for (uint32_t i = 0; i < N; ++i) o << "    double " << ub(i) << " = lam[" << i << "] * hm;\n";
             for (uint32_t k = 0; k < d.n_ops; ++k)
                 if (!alias[N + k]) o << "    double " << ub(N + k) << " = 0.0;\n";
@@ -1422,10 +1430,10 @@ struct Gen {
         o << "static __device__ __noinline__ void hyk_jets_bw(double *__restrict__ S, const double t0, const double h, "
              "double *__restrict__ lam, double *__restrict__ pb) {\n";
         // x̄_p comes from the Horner update only
-        o << "    double hp = 1.0;\n";
-        for (uint32_t q = 0; q < p; ++q) o << "    hp = hp * h;\n";
-        for (uint32_t i = 0; i < N; ++i) o << "    " << smem((uint32_t)akslot[i]) << " = lam[" << i << "] * hp;\n";
-        for (uint32_t mm = p; mm-- > 0;) o << "    hyk_bw_o" << mm << "(S, t0, h, lam, pb);\n";
+        o << "    double hp[" << p + 1 << "];\n    hp[0] = 1.0;\n";
+        for (uint32_t q = 0; q < p; ++q) o << "    hp[" << q + 1 << "] = hp[" << q << "] * h;\n";
+        for (uint32_t i = 0; i < N; ++i) o << "    " << smem((uint32_t)akslot[i]) << " = lam[" << i << "] * hp[" << p << "];\n";
+        for (uint32_t mm = p; mm-- > 0;) o << "    hyk_bw_o" << mm << "(S, t0, hp[" << mm << "], lam, pb);\n";
         o << "}\n";
     }
 };
