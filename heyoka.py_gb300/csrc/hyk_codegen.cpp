@@ -1493,6 +1493,9 @@ struct TeamGen {
     // members, one per round of the team, in registers over all orders.
     uint32_t T = 0;
     std::map<const Group *, uint32_t> rounds;
+    // Powers whose products with the coefficients n alpha - j (alpha + 1) are
+    // spread over the team (spread_powers): the first slot of the products.
+    std::map<const Group *, uint32_t> spread;
 
     TeamGen(const Dec &dd, uint32_t order, bool cold_rows = false)
         : g(dd, order, false, false), d(dd), p(order), N(dd.n_eq), NU(dd.n_u()) {
@@ -1712,6 +1715,7 @@ struct TeamGen {
                     D.kc = tkslot[u];
                     D.inv = tislot[u];
                     if (op.op == HYK_OP_SIN || op.op == HYK_OP_COS) D.prt = tslot[op.aux];
+                    if (op.op == HYK_OP_POW) D.x3 = (int)(descs.size() - gr.off);  // the member's number
                     if (A.kind == HYK_ARG_NUM) D.num = A.num;
                     if (B.kind == HYK_ARG_NUM && op.op != HYK_OP_POW) D.num = B.num;
                     if (g.fused(u)) {
@@ -1780,6 +1784,43 @@ struct TeamGen {
         return busy > 0 ? work / busy : 0.0;
     }
 
+    // The team's FP64 instructions of one order over those of one thread (the mean
+    // over the orders: p / 2 terms a convolution, half as many per leaf of a sum
+    // of squares, two instructions a term of a power, whose products may be
+    // spread over the team).
+    double instr(uint32_t team) const {
+        double one = 0, all = 0;
+        const double h = 0.5 * p;
+        auto add = [&](double m, double w) {
+            one += m * w;
+            all += std::ceil(m / team) * w;
+        };
+        for (auto &lv : levels)
+            for (auto &gr : lv) {
+                const uint32_t u = gr.members[0];
+                const auto &op = d.ops[u - N];
+                const Ref A = g.res(op.a), B = g.res(op.b);
+                const double m = (double)gr.members.size();
+                if (g.cst[u]) continue;
+                if (g.fused_sq(u)) {
+                    add(m, 0.5 * h * (double)g.fz_x(u).size() + 1.0);
+                } else if (g.fused_sc(u)) {
+                    add(m, (double)g.fz_x(u).size());
+                } else if (op.op == HYK_OP_ADD || op.op == HYK_OP_SUB || op.op == HYK_OP_NEG ||
+                           (op.op == HYK_OP_MUL && !(isU(A) && isU(B)))) {
+                    add(m, 1.0);
+                } else if (op.op == HYK_OP_POW) {
+                    add(m, h + 2.0);
+                    one += m * h;
+                    all += spread_need((uint32_t)m, team, p) ? std::ceil(m * h / team) : std::ceil(m / team) * h;
+                } else {
+                    add(m, op.op == HYK_OP_SQUARE ? 0.5 * h + 1.0 : h + 1.0);
+                }
+            }
+        for (auto &gr : supd) add((double)gr.members.size(), 1.0);
+        return one > 0 ? all / one : 1.0;
+    }
+
     // ---- expressions (D = the thread's descriptor, n = the order)
     static std::string wrap(const Ref &r, const std::string &s) { return r.neg ? "(-" + s + ")" : s; }
     // The current order of u-variable u (not time-constant) whose slot is in
@@ -1830,6 +1871,51 @@ struct TeamGen {
         else
             v = lit(0.0);
         out(u, n0, v);
+    }
+
+    // A group of few powers leaves most of the team idle along two
+    // instructions per term: the product of the coefficient with a lower order
+    // of the base, and the multiply-add. The products of order n need orders up
+    // to n - 1 only, so the whole team forms them at the start of the order, in
+    // slots of their own, when the powers are at most a quarter of the team.
+    // A lone warp is bound by its instructions there, and the integer products of
+    // the lane form cost it as much as they save.  1003 Kepler orbits to t = 50,
+    // teams of 8 and 16: 39.2 -> 35.1 and 38.7 -> 34.6 ms (of 4: 36.9 -> 36.8);
+    // 3001 variational ones, teams of 16: 37.4 -> 34.5 ms.
+    static uint32_t spread_need(uint32_t members, uint32_t team, uint32_t p) {
+        return p > 2 && 4 * members <= team ? members * (p - 2) : 0;
+    }
+    void spread_powers(uint32_t team) {
+        for (auto &lv : levels)
+            for (auto &gr : lv) {
+                const uint32_t u = gr.members[0];
+                if (g.fused(u) || g.cst[u] || d.ops[u - N].op != HYK_OP_POW) continue;
+                const uint32_t need = spread_need((uint32_t)gr.members.size(), team, p);
+                if (!need) continue;
+                spread[&gr] = nslot;
+                nslot += need;
+            }
+    }
+    size_t alpha_index(double alpha) const {
+        size_t ai = 0;
+        while (ai < alphas.size() && std::memcmp(&alphas[ai], &alpha, sizeof alpha) != 0) ++ai;
+        return ai;
+    }
+    void emit_spread() {
+        if (spread.empty()) return;
+        for (auto &lv : levels)
+            for (auto &gr : lv) {
+                auto it = spread.find(&gr);
+                if (it == spread.end()) continue;
+                const uint32_t u = gr.members[0], m = (uint32_t)gr.members.size();
+                const std::string pc = "hyk_pc" + std::to_string(alpha_index(d.ops[u - N].b.num));
+                o << "#pragma unroll 1\n        for (int e = r; e < " << m << " * (n - 1); e += HYK_TEAM) {\n";
+                o << "            const hyk_tdesc &D = hyk_td[" << gr.off << " + " << (m > 1 ? "e % " + std::to_string(m) : "0")
+                  << "];\n            const int j = 1 + e" << (m > 1 ? " / " + std::to_string(m) : "") << ";\n";
+                o << "            S[" << it->second << " + e] = HYK_MUL(" << pc << "[n * (HYK_ORDER + 1) + j], "
+                  << at(opnds(u).first, 'a', "n - j") << ");\n        }\n";
+            }
+        o << "        __syncwarp();\n";
     }
 
     // The groups whose rounds are emitted one after the other instead of as a
@@ -2157,6 +2243,16 @@ struct TeamGen {
             };
             // (the products in integer arithmetic: see the lane form; 65536
             // six-body members over a grid 245.7 -> 240.3 ms)
+            const auto sp = spread.find(&gr);
+            if (sp != spread.end()) {
+                const uint32_t m = (uint32_t)gr.members.size();
+                const std::string t = "S[" + std::to_string(sp->second) + " + (j - 1) * " + std::to_string(m) + " + D.x3]";
+                o << "            hyk_real acc = HYK_MUL(HYK_MUL(" << pc << "], " << at(A, 'a', "n") << "), S[D.c]);\n";
+                o << "#pragma unroll " << ju << "\n";
+                o << "            for (int j = 1; j < n; ++j) acc = " << fma_ << "(" << t << ", S[D.c + j], acc);\n";
+                out(u, false, "HYK_MUL(HYK_MUL(acc, hyk_invn[n]), S[D.inv])");
+                break;
+            }
             const bool ints = int_coefs(op.b.num);
             o << "            hyk_real acc;\n";
             if (ints) o << "            unsigned bad = 0;\n";
@@ -2255,6 +2351,7 @@ struct TeamGen {
     }
 
     void emit_order(bool n0) {
+        if (!n0) emit_spread();
         for (auto &lv : levels) {
             for (auto &gr : lv) emit_group_op(gr, n0);
             o << "        __syncwarp();\n";
@@ -2447,10 +2544,25 @@ bool team_layout(const Dec &d, uint32_t order, TeamInfo &info, std::string &err)
         err = tg.err;
         return false;
     }
+    info.n_raw = tg.nslot;
     info.n_slot = tg.nslot | 1u;
-    for (uint32_t T = 1; T <= 32; T *= 2) info.util[__builtin_ctz(T)] = tg.util(T);
+    for (uint32_t T = 1; T <= 32; T *= 2) {
+        uint32_t extra = 0;
+        for (auto &lv : tg.levels)
+            for (auto &gr : lv) {
+                const uint32_t u = gr.members[0];
+                if (!tg.g.fused(u) && !tg.g.cst[u] && d.ops[u - d.n_eq].op == HYK_OP_POW)
+                    extra += TeamGen::spread_need((uint32_t)gr.members.size(), T, order);
+            }
+        info.n_spread[__builtin_ctz(T)] = extra;
+    }
+    for (uint32_t T = 1; T <= 32; T *= 2) {
+        info.util[__builtin_ctz(T)] = tg.util(T);
+        info.instr[__builtin_ctz(T)] = tg.instr(T);
+    }
     TeamGen tc(d, order, true);
     info.n_slot_cold = (tc.cold && tc.analyse()) ? (tc.nslot | 1u) : 0;
+    info.n_raw_cold = info.n_slot_cold ? tc.nslot : 0;
     return true;
 }
 
@@ -2471,6 +2583,7 @@ bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, si
         return false;
     }
     tg.g.emit_jets();  // flop count of the same recurrences
+    tg.spread_powers(team);
     tg.plan_rounds(team);
     const double p = (double)order;
     const double rhofac = rhofac_of(order);

@@ -61,6 +61,11 @@ struct TeamInfo {
     uint32_t n_slot = 0;       // doubles per trajectory (padded)
     uint32_t n_slot_cold = 0;  // the same with cold state rows (0: the system has none)
     double util[6] = {0, 0, 0, 0, 0, 0};
+    double instr[6] = {1, 1, 1, 1, 1, 1};  // FP64 instructions of a team's warp over those of one thread
+    uint32_t n_spread[6] = {0, 0, 0, 0, 0, 0};  // doubles more for the powers' products spread over the team
+    uint32_t n_raw = 0, n_raw_cold = 0;         // n_slot and n_slot_cold before the padding to an odd number
+    // Doubles per trajectory of a team of T threads (odd).
+    uint32_t slots(uint32_t T, bool cold) const { return ((cold ? n_raw_cold : n_raw) + n_spread[__builtin_ctz(T)]) | 1u; }
 };
 // false (with the reason) when an operation has no team-form code.
 bool team_layout(const Dec &d, uint32_t order, TeamInfo &info, std::string &err);

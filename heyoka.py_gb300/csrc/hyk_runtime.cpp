@@ -333,54 +333,50 @@ static uint32_t default_team(const hyk::TeamInfo &ti, size_t lane_bytes, size_t 
 // the time of one step of all of them in units of a lane-form step's FP64
 // instructions, 64 cycles each whatever the active lanes of the warp.
 //
-// A team of T threads issues 1 / (T util) of them; a warp alone on its
-// sub-partition takes c times its FP64 time (1.15 measured for the lane form,
-// 1.55 for teams), and w warps on one (c^4 + w^4)^(1/4), w at most what is
+// A team of T threads issues a share of them (TeamInfo::instr); a warp alone on
+// its sub-partition takes c times its FP64 time (1.15 measured for the lane form,
+// 1.6 for teams), and w warps on one (c^4 + w^4)^(1/4), w at most what is
 // resident.  Trajectories of one batch end at different times, so that the warps
 // at work are counted at 0.7 of those at the start.  A small batch cannot fill
 // the warps of the lane form, so a team that spreads each trajectory wins
 // there.  Measured, us a step (estimated, in lane-form steps): 331 six-body
-// members with teams of 32 and 16 69 and 100 (0.082, 0.109), 3001 of them 249 and
-// 185 (0.185, 0.138); Kepler in the lane form and with teams of 4 59 and 47 for
-// 1003 orbits (1.15, 0.88), 59 and 53 for 10007 (1.15, 1.02), 59 and 83 for 20011
-// (1.15, 1.67).  Lane-form systems so large that their recurrences are split into
+// members with teams of 32 and 16 69 and 100 (0.089, 0.114), 3001 of them 249 and
+// 185 (0.195, 0.142); 1003 Kepler orbits in the lane form and with teams of 4, 8
+// and 16 59, 46, 44 and 43 (1.15, 0.92, 0.90, 0.87), 20011 in the lane form and
+// with teams of 4 59 and 83 (1.15, 1.69); CR3BP 96 and 95 with teams of 8 (1.15,
+// 1.28).  Lane-form systems so large that their recurrences are split into
 // functions and still spill are counted at c = 4 (first-order variational Kepler,
 // 42 equations: 2.05 ms a step in the lane form, 127 us with teams of 32; ptxas
 // 41 s and 0.8 s).  The default form is kept unless another is estimated 5 %
-// faster, and of teams within 12 % of the fastest the one with the fewest
-// instructions is taken, the smallest if several have as few: the last
-// trajectories then run fastest (3001 variational Kepler orbits with teams of 8
-// and 16 12.6 and 11.8 ms; 1003 Kepler orbits with 4 and 16 3.49 and 3.73 ms).
+// faster, and of teams within 8 % of the fastest the one with the fewest
+// instructions is taken: the last trajectories then run fastest.
 static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool large, size_t real_bytes, const Device &dv,
                                uint64_t n) {
     const double smsp = 4.0 * dv.n_sm;
     auto cost = [&](double c, double warps, double resident) {
         const double w = 0.7 * warps / smsp, k = std::min(resident, w);
-        const double t = w <= 1.0 ? c : std::pow(c * c * c * c + k * k * k * k, 0.25);
-        return t * std::max(1.0, w / std::max(k, 1.0));
+        const double t = k <= 1.0 ? c : std::pow(c * c * c * c + k * k * k * k, 0.25);
+        return t * std::max(1.0, w / std::max(k, 1e-9));
     };
-    double c[6], instr[6];
+    double c[6];
     c[0] = cost(large ? 4.0 : 1.15, (double)n / 32.0, 2.0);
-    instr[0] = 1.0;
     for (uint32_t l = 1; l <= 5; ++l) {
         const uint32_t T = 1u << l;
-        const uint32_t slots = ti.n_slot_cold ? ti.n_slot_cold : ti.n_slot;
-        const size_t cta = (size_t)(32 / T) * slots * real_bytes;
+        const size_t cta = (size_t)(32 / T) * ti.slots(T, ti.n_slot_cold != 0) * real_bytes;
         c[l] = INFINITY;
-        instr[l] = 1.0 / (T * ti.util[l]);
         if (cta > (size_t)dv.smem_optin) continue;
         const double resident = std::min(16.0, (double)((size_t)dv.smem_per_sm / (cta + 1024))) / 4.0;
-        c[l] = cost(1.55, (double)n * T / 32.0, resident) * instr[l];
+        c[l] = cost(1.6, (double)n * T / 32.0, resident) * ti.instr[l];
     }
     const uint32_t dl = dflt ? (uint32_t)__builtin_ctz(dflt) : 0;
     uint32_t best = 0;
     for (uint32_t l = 1; l <= 5; ++l)
         if (c[l] < c[best]) best = l;
-    if (best == 0 || c[best] * 1.05 >= c[dl]) return c[best] * 1.05 < c[dl] ? 0 : dflt;
+    if (c[best] * 1.05 >= c[dl]) return dflt;
     uint32_t pick = best;
     for (uint32_t l = 1; l <= 5; ++l)
-        if (c[l] <= 1.12 * c[best] && instr[l] < 0.98 * instr[pick]) pick = l;
-    return 1u << pick;
+        if (best && c[l] <= 1.08 * c[best] && ti.instr[l] < 0.98 * ti.instr[pick]) pick = l;
+    return pick ? 1u << pick : 0;
 }
 
 extern "C" {
@@ -453,7 +449,7 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     }
     if (m->team) {
         if (blk == 0) blk = 32;
-        nslot = ti.n_slot;
+        nslot = ti.slots(m->team, false);
         lane_bytes = (size_t)nslot * real_bytes;
     }
     // Lane form of a system whose coefficients do not fit 32 lanes of shared
@@ -483,11 +479,11 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
         // trajectories instead of six).
         if (!m->gmem && ti.n_slot_cold && !(m->cfg.flags & HYK_CFG_NO_COLD_ROWS)) {
             const size_t tpc = blk / m->team;
-            const size_t hot = tpc * ti.n_slot * real_bytes, cold = tpc * ti.n_slot_cold * real_bytes;
+            const size_t hot = tpc * ti.slots(m->team, false) * real_bytes, cold = tpc * ti.slots(m->team, true) * real_bytes;
             const uint32_t ch = hot > (size_t)dv.smem_optin ? 0 : (uint32_t)((size_t)dv.smem_per_sm / (hot + 1024));
             const uint32_t cc = cold > (size_t)dv.smem_optin ? 0 : (uint32_t)((size_t)dv.smem_per_sm / (cold + 1024));
             if (std::min<uint32_t>(cc, 32) > std::min<uint32_t>(ch, 32)) {
-                nslot = ti.n_slot_cold;
+                nslot = ti.slots(m->team, true);
                 lane_bytes = (size_t)nslot * real_bytes;
                 m->ncold = m->d.n_eq;
                 m->cold_ctas = (int)std::min<uint32_t>(cc, 32);
@@ -739,7 +735,7 @@ int hyk_config_for(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t *c
     // state rows does without them (331 six-body members: teams of 32 87 us a
     // step with them, 76 without; teams of 16 124 and 99).
     if (team && ti.n_slot_cold) {
-        const size_t cta = (size_t)(32 / team) * ti.n_slot * sizeof(double);
+        const size_t cta = (size_t)(32 / team) * ti.slots(team, false) * sizeof(double);
         const uint64_t ctas = cta > (size_t)dv->smem_optin ? 0 : std::min<uint64_t>(24, (size_t)dv->smem_per_sm / (cta + 1024));
         if (n_lanes <= ctas * dv->n_sm * (32 / team)) c.flags |= HYK_CFG_NO_COLD_ROWS;
     }
