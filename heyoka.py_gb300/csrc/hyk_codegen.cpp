@@ -1496,6 +1496,17 @@ struct TeamGen {
     // Powers whose products with the coefficients n alpha - j (alpha + 1) are
     // spread over the team (spread_powers): the first slot of the products.
     std::map<const Group *, uint32_t> spread;
+    // Small systems: the orders one after the other with every trip count a
+    // constant (no loop control, no address arithmetic: every operand is the
+    // descriptor's slot and an immediate), instead of a loop over the orders.
+    // A lone warp is bound by those instructions: 1003 Kepler orbits to t = 50
+    // 34.9 -> 31.7 ms, CR3BP with teams of 16 95 -> 86 us a step.  Above kFullOps the
+    // gain is small and the code long (six bodies over a grid 210 -> 206 ms, ptxas
+    // 0.7 -> 5 s).
+    static constexpr uint32_t kFullOps = 1000;
+    static bool is_full(const Dec &dd, uint32_t order) { return (uint64_t)dd.n_ops * order <= kFullOps; }
+    bool full = false;
+    std::string unroll(int k) const { return full ? "#pragma unroll\n" : "#pragma unroll " + std::to_string(k) + "\n"; }
 
     TeamGen(const Dec &dd, uint32_t order, bool cold_rows = false)
         : g(dd, order, false, false), d(dd), p(order), N(dd.n_eq), NU(dd.n_u()) {
@@ -2015,7 +2026,7 @@ struct TeamGen {
         for (uint32_t c = 0; c < R; ++c)
             o << "            hyk_real acc" << c << " = HYK_MUL(" << in_round(gr, c, at(A, 'a', "0")) << ", "
               << in_round(gr, c, at(B, 'b', "n")) << ");\n";
-        o << "#pragma unroll " << (R > 1 ? 2 : ju) << "\n            for (int j = 1; j <= n; ++j) {\n";
+        o << unroll(R > 1 ? 2 : ju) << "            for (int j = 1; j <= n; ++j) {\n";
         for (uint32_t c = 0; c < R; ++c)
             o << "                acc" << c << " = HYK_FMA(" << in_round(gr, c, at(A, 'a', "j")) << ", "
               << in_round(gr, c, at(B, 'b', "n - j")) << ", acc" << c << ");\n";
@@ -2094,7 +2105,7 @@ struct TeamGen {
                         o << "            hyk_real acc = HYK_MUL(" << lx(0, "0") << ", " << lx(0, "n") << ");\n";
                     else
                         o << "            acc = " << fma_ << "(" << lx(i, "0") << ", " << lx(i, "n") << ", acc);\n";
-                    o << "#pragma unroll " << ju << "\n";
+                    o << unroll(ju);
                     o << "            for (int j = 1; 2 * j < n; ++j) acc = " << fma_ << "(" << lx(i, "j") << ", "
                       << lx(i, "n - j") << ", acc);\n";
                 }
@@ -2166,7 +2177,7 @@ struct TeamGen {
         case HYK_OP_MUL:
             if (isU(A) && isU(B)) {
                 o << "            hyk_real acc = HYK_MUL(" << at(A, 'a', "0") << ", " << at(B, 'b', "n") << ");\n";
-                o << "#pragma unroll " << ju << "\n";
+                o << unroll(ju);
                 o << "            for (int j = 1; j <= n; ++j) acc = " << fma_ << "(" << at(A, 'a', "j") << ", "
                   << at(B, 'b', "n - j") << ", acc);\n";
                 out(u, false, "acc");
@@ -2193,7 +2204,7 @@ struct TeamGen {
         case HYK_OP_DIV:
             if (isU(B)) {
                 o << "            hyk_real acc = HYK_MUL(" << at(B, 'b', "1") << ", S[D.c + n - 1]);\n";
-                o << "#pragma unroll " << ju << "\n";
+                o << unroll(ju);
                 o << "            for (int j = 2; j <= n; ++j) acc = " << fma_ << "(" << at(B, 'b', "j")
                   << ", S[D.c + n - j], acc);\n";
                 const std::string a = isU(A) ? cur(A, 'a', false) : lit(0.0);
@@ -2204,7 +2215,7 @@ struct TeamGen {
             break;
         case HYK_OP_SQUARE:
             o << "            hyk_real acc = HYK_MUL(" << at(A, 'a', "0") << ", " << at(A, 'a', "n") << ");\n";
-            o << "#pragma unroll " << ju << "\n";
+            o << unroll(ju);
             o << "            for (int j = 1; 2 * j < n; ++j) acc = " << fma_ << "(" << at(A, 'a', "j") << ", "
               << at(A, 'a', "n - j") << ", acc);\n";
             o << "            acc = HYK_ADD(acc, acc);\n";
@@ -2218,7 +2229,7 @@ struct TeamGen {
             o << "                acc = HYK_MUL(S[D.c + 1], S[D.c + 1]);\n";
             o << "            } else if (n > 2) {\n";
             o << "                acc = HYK_MUL(S[D.c + 1], S[D.c + n - 1]);\n";
-            o << "#pragma unroll " << ju << "\n";
+            o << unroll(ju);
             o << "                for (int j = 2; 2 * j < n; ++j) acc = " << fma_ << "(S[D.c + j], S[D.c + n - j], acc);\n";
             o << "                acc = HYK_ADD(acc, acc);\n";
             o << "                if ((n & 1) == 0) acc = " << fma_ << "(S[D.c + n / 2], S[D.c + n / 2], acc);\n";
@@ -2233,7 +2244,7 @@ struct TeamGen {
             const std::string pc = "hyk_pc" + std::to_string(ai) + "[n * (HYK_ORDER + 1)";
             auto chain = [&](bool ints) {
                 o << "            acc = HYK_MUL(HYK_MUL(" << pc << "], " << at(A, 'a', "n") << "), S[D.c]);\n";
-                o << "#pragma unroll " << ju << "\n";
+                o << unroll(ju);
                 o << "            for (int j = 1; j < n; ++j) acc = " << fma_ << "(";
                 if (ints)
                     o << "HYK_MULK(" << at(A, 'a', "n - j") << ", hyk_pk" << ai << "[n * (HYK_ORDER + 1) + j], &bad)";
@@ -2248,7 +2259,7 @@ struct TeamGen {
                 const uint32_t m = (uint32_t)gr.members.size();
                 const std::string t = "S[" + std::to_string(sp->second) + " + (j - 1) * " + std::to_string(m) + " + D.x3]";
                 o << "            hyk_real acc = HYK_MUL(HYK_MUL(" << pc << "], " << at(A, 'a', "n") << "), S[D.c]);\n";
-                o << "#pragma unroll " << ju << "\n";
+                o << unroll(ju);
                 o << "            for (int j = 1; j < n; ++j) acc = " << fma_ << "(" << t << ", S[D.c + j], acc);\n";
                 out(u, false, "HYK_MUL(HYK_MUL(acc, hyk_invn[n]), S[D.inv])");
                 break;
@@ -2272,7 +2283,7 @@ struct TeamGen {
                 break;
             }
             o << "            hyk_real acc = HYK_MUL(" << wrap(A, "S[D.ka]") << ", S[D.c + n - 1]);\n";
-            o << "#pragma unroll " << ju << "\n";
+            o << unroll(ju);
             o << "            for (int j = 2; j <= n; ++j) acc = " << fma_ << "(" << wrap(A, "S[D.ka + j - 1]")
               << ", S[D.c + n - j], acc);\n";
             out(u, false, "HYK_MUL(acc, hyk_invn[n])");
@@ -2281,7 +2292,7 @@ struct TeamGen {
             o << "            hyk_real acc = " << lit(0.0) << ";\n";
             o << "            if (n >= 2) {\n";
             o << "                acc = HYK_MUL(S[D.kc], " << at(A, 'a', "n - 1") << ");\n";
-            o << "#pragma unroll " << ju << "\n";
+            o << unroll(ju);
             o << "                for (int j = 2; j < n; ++j) acc = " << fma_ << "(S[D.kc + j - 1], " << at(A, 'a', "n - j")
               << ", acc);\n";
             o << "            }\n";
@@ -2294,7 +2305,7 @@ struct TeamGen {
                 o << "            const hyk_real acc = " << lit(1.0) << " * S[D.prt + n - 1];\n";
             } else {
                 o << "            hyk_real acc = HYK_MUL(" << wrap(A, "S[D.ka]") << ", S[D.prt + n - 1]);\n";
-                o << "#pragma unroll " << ju << "\n";
+                o << unroll(ju);
                 o << "            for (int j = 2; j <= n; ++j) acc = " << fma_ << "(" << wrap(A, "S[D.ka + j - 1]")
                   << ", S[D.prt + n - j], acc);\n";
             }
@@ -2411,10 +2422,18 @@ struct TeamGen {
         o << "    {\n        // ---- order 0\n";
         emit_order(true);
         o << "    }\n";
-        o << "#pragma unroll 1\n";
-        o << "    for (int n = 1; n < HYK_ORDER; ++n) {\n";
-        emit_order(false);
-        o << "    }\n";
+        if (full) {
+            for (uint32_t k = 1; k < p; ++k) {
+                o << "    {\n        constexpr int n = " << k << ";\n";
+                emit_order(false);
+                o << "    }\n";
+            }
+        } else {
+            o << "#pragma unroll 1\n";
+            o << "    for (int n = 1; n < HYK_ORDER; ++n) {\n";
+            emit_order(false);
+            o << "    }\n";
+        }
         o << "}\n";
     }
 };
@@ -2545,6 +2564,7 @@ bool team_layout(const Dec &d, uint32_t order, TeamInfo &info, std::string &err)
         return false;
     }
     info.n_raw = tg.nslot;
+    info.unrolled = TeamGen::is_full(d, order);
     info.n_slot = tg.nslot | 1u;
     for (uint32_t T = 1; T <= 32; T *= 2) {
         uint32_t extra = 0;
@@ -2585,6 +2605,7 @@ bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, si
     tg.g.emit_jets();  // flop count of the same recurrences
     tg.spread_powers(team);
     tg.plan_rounds(team);
+    tg.full = TeamGen::is_full(d, order);
     const double p = (double)order;
     const double rhofac = rhofac_of(order);
     const uint32_t nt = tg.nslot | 1u;
@@ -2652,6 +2673,7 @@ bool generate_host(const Dec &d, uint32_t order, bool adjoint, std::string &src,
             h << "#define HYK_SX(i, n) S[(i) * HYK_XS + (n)]\n";
         h << "#define HYK_PAR(k) S[HYK_PAR_SLOT + (k)]\n";
         tg.plan_rounds(1);
+        tg.full = TeamGen::is_full(d, order);
         tg.emit();
         h << tg.o.str();
         h << "extern \"C\" int hyk_host_nslot(void) { return HYK_NSLOT; }\n";

@@ -335,16 +335,16 @@ static uint32_t default_team(const hyk::TeamInfo &ti, size_t lane_bytes, size_t 
 //
 // A team of T threads issues a share of them (TeamInfo::instr); a warp alone on
 // its sub-partition takes c times its FP64 time (1.15 measured for the lane form,
-// 1.6 for teams), and w warps on one (c^4 + w^4)^(1/4), w at most what is
+// 1.6 for teams, 1.35 with the orders unrolled), and w warps on one (c^4 + w^4)^(1/4), w at most what is
 // resident.  Trajectories of one batch end at different times, so that the warps
 // at work are counted at 0.7 of those at the start.  A small batch cannot fill
 // the warps of the lane form, so a team that spreads each trajectory wins
 // there.  Measured, us a step (estimated, in lane-form steps): 331 six-body
 // members with teams of 32 and 16 69 and 100 (0.089, 0.114), 3001 of them 249 and
-// 185 (0.195, 0.142); 1003 Kepler orbits in the lane form and with teams of 4, 8
-// and 16 59, 46, 44 and 43 (1.15, 0.92, 0.90, 0.87), 20011 in the lane form and
-// with teams of 4 59 and 83 (1.15, 1.69); CR3BP 96 and 95 with teams of 8 (1.15,
-// 1.28).  Lane-form systems so large that their recurrences are split into
+// 185 (0.195, 0.142); 1003 Kepler orbits in the lane form and with teams of 4
+// and 16 59, 42 and 39 (1.15, 0.77, 0.74), 10007 in the lane form and with teams
+// of 4 59 and 50 (1.15, 0.95); 1003 CR3BP trajectories in the lane form and with
+// teams of 16 96 and 86 (1.15, 1.06).  Lane-form systems so large that their recurrences are split into
 // functions and still spill are counted at c = 4 (first-order variational Kepler,
 // 42 equations: 2.05 ms a step in the lane form, 127 us with teams of 32; ptxas
 // 41 s and 0.8 s).  The default form is kept unless another is estimated 5 %
@@ -366,7 +366,7 @@ static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool larg
         c[l] = INFINITY;
         if (cta > (size_t)dv.smem_optin) continue;
         const double resident = std::min(16.0, (double)((size_t)dv.smem_per_sm / (cta + 1024))) / 4.0;
-        c[l] = cost(1.6, (double)n * T / 32.0, resident) * ti.instr[l];
+        c[l] = cost(ti.unrolled ? 1.35 : 1.6, (double)n * T / 32.0, resident) * ti.instr[l];
     }
     const uint32_t dl = dflt ? (uint32_t)__builtin_ctz(dflt) : 0;
     uint32_t best = 0;
