@@ -957,6 +957,7 @@ struct Gen {
     // State variable i, order n in the jets code: shared memory, or for a
     // cold row (n >= 1) the module's global buffer.
     std::string sx(uint32_t i, uint32_t n) const {
+        if (inreg) return "hyk_x[" + std::to_string(i) + "][" + std::to_string(n) + "]";
         if (coldrows && crow[i] >= 0 && n > 0)
             return "HYK_CX(" + std::to_string(crow[i] * p + n - 1) + ")";
         return "HYK_SX(" + std::to_string(i) + ", " + std::to_string(n) + ")";
@@ -988,10 +989,17 @@ struct Gen {
         std::string coldg = coldrows ? "    hyk_real *__restrict__ hyk_cold_g = hyk_cold_ptr();\n" : "";
         if (fmaops()) coldg += "    HYK_FMAOPS_CONSTS\n";
         if (!split) {
-            o << "static __device__ __noinline__ void hyk_jets(hyk_real *__restrict__ S, const hyk_real t0, "
-                 "const unsigned hyk_wm = 0xffffffffu) {\n" << coldg;
+            if (inreg)
+                o << "static __device__ __forceinline__ void hyk_jets(hyk_real *__restrict__ S, hyk_rows &hyk_x, const hyk_real t0, "
+                     "const unsigned hyk_wm = 0xffffffffu) {\n" << coldg;
+            else
+                o << "static __device__ __noinline__ void hyk_jets(hyk_real *__restrict__ S, const hyk_real t0, "
+                     "const unsigned hyk_wm = 0xffffffffu) {\n" << coldg;
             if (inreg) o << "    HYK_WARP_SYNC();\n";  // reconverge once: nothing is re-read between the orders
-            for (uint32_t i = 0; i < N; ++i) o << "    const hyk_real " << vname(i, 0) << " = HYK_SX(" << i << ", 0);\n";
+            for (uint32_t i = 0; i < N; ++i) {
+                o << "    const hyk_real " << vname(i, 0) << " = HYK_SX(" << i << ", 0);\n";
+                if (inreg) o << "    hyk_x[" << i << "][0] = " << vname(i, 0) << ";\n";
+            }
         }
         const uint32_t last = evx ? p : p - 1;  // order p: the event functions' cone only
         for (uint32_t n = 0; n <= last; ++n) {
@@ -2476,12 +2484,9 @@ uint32_t count_slots(const Dec &d, uint32_t order, bool adjoint, bool pin, bool 
     return g.nslot;
 }
 
-// The step-size rule's rho: of one logarithm in double precision, with the
-// same bits as hyk_dm_rho (hyk_rho_one in kernel_common.inc).
-static std::string rho_macro(bool f32) {
-    if (f32) return "#define HYK_RHO(mp, mq, num) HYK_DM_RHO((mp), (mq), (num), HYK_INV_P, HYK_INV_PM1)\n";
-    return "#define HYK_RHO_ONE 1\n#define HYK_RHO(mp, mq, num) hyk_rho_one((mp), (mq), (num))\n";
-}
+// The step-size rule's rho: of one logarithm, with the same bits as hyk_dm_rho
+// (hyk_rho_one in kernel_common.inc).
+static std::string rho_macro() { return "#define HYK_RHO_ONE 1\n#define HYK_RHO(mp, mq, num) hyk_rho_one((mp), (mq), (num))\n"; }
 
 struct PrecisionScope {
     explicit PrecisionScope(bool f32) { g_f32 = f32; }
@@ -2519,9 +2524,10 @@ bool generate(const Dec &d, uint32_t order, bool pin_arith, uint32_t blk, size_t
              "? 1.0 / pow((mq) / (num), HYK_INV_PM1) : 1.0 / pow((mp) / (num), HYK_INV_P))\n";
     } else {
         h << "#define HYK_FMA_ACC(a, b, c) HYK_FMA((a), (b), (c))\n";
-        h << rho_macro(f32);
+        h << rho_macro();
     }
     h << "#define HYK_LB __launch_bounds__(HYK_TPB" << (g.inreg && min_ctas ? ", " + std::to_string(min_ctas) : "") << ")\n";
+    h << "#define HYK_INREG " << (g.inreg ? 1 : 0) << "\n";
     if (adjoint) h << "#define HYK_ADJOINT 1\n";
     h << "#define HYK_HIGH_ACC " << (high_acc ? 1 : 0) << "\n";
     if (g.coldrows) h << "#define HYK_CSTRIDE " << cold_stride << "ULL\n";
@@ -2620,7 +2626,7 @@ bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, si
       << lit(recip(p - 1.0)) << "\n";
     h << precision_header(false);
     h << "#define HYK_FMA_ACC(a, b, c) HYK_FMA((a), (b), (c))\n";
-    h << rho_macro(f32);
+    h << rho_macro();
     h << "#define HYK_NEV 0\n#define HYK_NTEV 0\n#define HYK_HIGH_ACC " << (high_acc ? 1 : 0) << "\n";
     h << kDmath << "\n";
     h << kCommon << "\n";

@@ -424,13 +424,14 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     } else if (want_team == 0 && team_ok) {
         m->team = default_team(ti, lane_bytes, real_bytes, dv);
     }
-    // Lane form of a small system: the histories in registers.  A term of a
-    // convolution then needs no shared-memory loads, which bound the float
-    // kernels (2^20 Kepler orbits, order 9, propagation kernel alone: 3.85 ms
-    // with two CTAs of 256 and the histories in shared memory, 3.34 with them
-    // in registers, 2.86 with the registers held to 80 so that six CTAs of 128
-    // share an SM) and lengthened the step of a warp alone on its FP64 unit
-    // (pendulum, order 20: 26 -> 24 us).
+    // Lane form of a small system: the histories in registers, and the state
+    // rows up to the state update.  A term of a convolution then needs no
+    // shared-memory loads, which bound the float kernels and lengthened the step of
+    // a warp alone on its FP64 unit.  2^20 Kepler orbits in float (order 9),
+    // propagation kernel alone: 3.85 ms with the histories in shared memory (two
+    // CTAs of 256), 2.86 with them in registers, 2.41 with the rows too, in ten
+    // CTAs of 64 and 96 registers a thread (six of 128 and 80 registers 2.66, five
+    // of 128 2.54).  Pendulum (order 20): 26, 24 and 22 us a step.
     const uint32_t n_live = !m->team && !pin && !adjoint && !(m->cfg.flags & HYK_CFG_GLOBAL_JETS)
                                 ? hyk::register_values(m->d, order, f32)
                                 : 0;
@@ -440,9 +441,10 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
         nslot = hyk::count_slots(m->d, order, false, false, false, nullptr, false, true);
         lane_bytes = (size_t)nslot * real_bytes;
         if (f32 && blk == 0) {
-            // about 34 registers besides the histories; at most 768 threads an SM
-            blk = 128;
-            const uint32_t regs = (n_live + 34 + 7) / 8 * 8;
+            // about 50 registers besides the histories (the rows of the other
+            // state variables among them); at most 768 threads an SM
+            blk = 64;
+            const uint32_t regs = (n_live + 50 + 7) / 8 * 8;
             min_ctas = std::min<uint32_t>(768, 65536 / regs) / blk;
             min_ctas = std::min<uint32_t>(min_ctas, (uint32_t)((size_t)dv.smem_per_sm / (blk * lane_bytes + 1024)));
         }
