@@ -222,14 +222,14 @@ double rhofac_of(uint32_t p) {
 std::string precision_header(bool pin) {
     std::string h;
     if (g_f32) {
-        h += "#define HYK_F32 1\n";
+        h += "#define HYK_F32 1\n#define HYK_NEG_IF(x, neg) HYK_DM_FFROM(HYK_DM_FBITS(x) ^ ((unsigned)(neg) << 31))\n";
         h += "#define HYK_FMA(a, b, c) __fmaf_rn((a), (b), (c))\n";
         h += "#define HYK_FMAOPS_CONSTS\n#define HYK_MUL(a, b) ((a) * (b))\n#define HYK_ADD(a, b) ((a) + (b))\n"
              "#define HYK_SUB(a, b) ((a) - (b))\n";
         h += "#define HYK_DM_EXP hyk_dmf_exp\n#define HYK_DM_LOG hyk_dmf_log\n#define HYK_DM_SINCOS hyk_dmf_sincos\n"
              "#define HYK_DM_POW hyk_dmf_pow\n#define HYK_DM_RHO hyk_dmf_rho\n";
     } else {
-        h += "#define HYK_F32 0\n";
+        h += "#define HYK_F32 0\n#define HYK_NEG_IF(x, neg) HYK_DM_FROM(HYK_DM_BITS(x) ^ ((unsigned long long)(neg) << 63))\n";
         h += "#define HYK_FMA(a, b, c) __fma_rn((a), (b), (c))\n";
         // x * y, x + y and x - y as fused multiply-adds (same bits); the
         // constants -0 and 1 come from volatile loads of module globals, so
@@ -1653,7 +1653,9 @@ struct TeamGen {
                 std::snprintf(buf, sizeof buf, "_a%a", op.b.num);
                 key += buf;
             }
-            if (op.op == HYK_OP_SIN || op.op == HYK_OP_COS) key += (u < (uint32_t)op.aux) ? "_lead" : "_follow";
+            // (sines and cosines in one group: the two of a pair are independent chains)
+            if (op.op == HYK_OP_SIN || op.op == HYK_OP_COS)
+                key = "opsc_" + rkey(A) + "_c" + (g.cst[u] ? "K" : (g.hist[u] ? "h" : "c")) + (g.needka[u] ? "k" : "");
             auto &lv = levels[level[u] - 1];
             auto &ix = index[level[u] - 1];
             auto it = ix.find(key);
@@ -1669,7 +1671,8 @@ struct TeamGen {
         std::map<std::string, size_t> sx;
         for (uint32_t i = 0; i < N; ++i) {
             const Ref R = g.res(d.rhs[i]);
-            const std::string key = "upd_" + rkey(R) + (g.needka[i] ? "k" : "");
+            // (variables of any kind and sign in one group: upd_operand)
+            const std::string key = "upd_" + (isU(R) ? std::string("v") : rkey(R)) + (g.needka[i] ? "k" : "");
             auto it = sx.find(key);
             if (it == sx.end()) {
                 sx[key] = supd.size();
@@ -1733,7 +1736,13 @@ struct TeamGen {
                     D.ka = isU(A) ? tkslot[A.u] : 0;
                     D.kc = tkslot[u];
                     D.inv = tislot[u];
-                    if (op.op == HYK_OP_SIN || op.op == HYK_OP_COS) D.prt = tslot[op.aux];
+                    if (op.op == HYK_OP_SIN || op.op == HYK_OP_COS) {
+                        // the partner's slot, whether this one evaluates the pair at
+                        // order 0 (the first of the two), whether it is the cosine
+                        D.prt = tslot[op.aux];
+                        D.b = u < (uint32_t)op.aux ? 1 : 0;
+                        D.inv = op.op == HYK_OP_COS ? 1 : 0;
+                    }
                     if (op.op == HYK_OP_POW) D.x3 = (int)(descs.size() - gr.off);  // the member's number
                     if (A.kind == HYK_ARG_NUM) D.num = A.num;
                     if (B.kind == HYK_ARG_NUM && op.op != HYK_OP_POW) D.num = B.num;
@@ -1768,6 +1777,10 @@ struct TeamGen {
                 D.c = tslot[i];
                 D.kc = tkslot[i];
                 if (R.kind == HYK_ARG_NUM) D.num = R.num;
+                if (isU(R)) {
+                    D.ka = coldvar(R.u) ? 1 : th(R.u) ? -1 : 0;
+                    D.prt = R.neg ? 1 : 0;
+                }
                 descs.push_back(D);
             }
         }
@@ -1978,7 +1991,7 @@ struct TeamGen {
                 if (g.needka[u]) ++ints;
                 c.push_back({&gr, conv, ((uint32_t)gr.members.size() + team - 1) / team, ints});
             }
-        for (auto &gr : supd) c.push_back({&gr, false, ((uint32_t)gr.members.size() + team - 1) / team, 3});
+        for (auto &gr : supd) c.push_back({&gr, false, ((uint32_t)gr.members.size() + team - 1) / team, 5});
         uint32_t left = kDescInts;
         for (const bool conv : {true, false})
             for (const Cand &x : c)
@@ -2156,12 +2169,9 @@ struct TeamGen {
                 break;
             case HYK_OP_SIN:
             case HYK_OP_COS:
-                if (u < (uint32_t)op.aux) {
-                    o << "            hyk_real sv, cv;\n";
-                    o << "            HYK_DM_SINCOS(" << a << ", &sv, &cv);\n";
-                    o << "            S[D.c] = " << (op.op == HYK_OP_SIN ? "sv" : "cv") << ";\n";
-                    o << "            S[D.prt] = " << (op.op == HYK_OP_SIN ? "cv" : "sv") << ";\n";
-                }
+                o << "            if (D.b) {\n                hyk_real sv, cv;\n";
+                o << "                HYK_DM_SINCOS(" << a << ", &sv, &cv);\n";
+                o << "                S[D.c] = D.inv ? cv : sv;\n                S[D.prt] = D.inv ? sv : cv;\n            }\n";
                 break;
             }
             return;
@@ -2317,11 +2327,20 @@ struct TeamGen {
                 o << "            for (int j = 2; j <= n; ++j) acc = " << fma_ << "(" << wrap(A, "S[D.ka + j - 1]")
                   << ", S[D.prt + n - j], acc);\n";
             }
-            out(u, false, op.op == HYK_OP_SIN ? "HYK_MUL(acc, hyk_invn[n])" : "(-HYK_MUL(acc, hyk_invn[n]))");
+            out(u, false, "hyk_flip(HYK_MUL(acc, hyk_invn[n]), D.inv)");
             break;
         }
     }
 
+    // The right-hand side's current order in an update, whatever its kind: from
+    // its history (mask -1), a cold state variable's two slots (1) or its only
+    // slot (0), with the sign of a folded negation.  One group for all updates:
+    // the six-body problem's 36 take three rounds of 16 threads, not two and two
+    // (65536 members' grid 210.2 -> 205.6 ms; the pendulum's two are one round of
+    // a team of two, its 1024 x 4 ensemble 79.3 -> 77.6 ms).
+    std::string upd_operand(bool n0) const {
+        return n0 ? "hyk_flip(S[D.a], D.prt)" : "hyk_flip(S[D.a + (n & D.ka)], D.prt)";
+    }
     void emit_group_upd(const Group &gr, bool n0) {
         o << "        // " << gr.key << "\n";
         if (!n0 && rounds.count(&gr)) {
@@ -2339,10 +2358,10 @@ struct TeamGen {
         const uint32_t i = gr.members[0];
         const Ref R = g.res(d.rhs[i]);
         std::string f;
-        if (n0) {
+        if (isU(R)) {
+            f = upd_operand(n0);
+        } else if (n0) {
             f = cur(R, 'a', true);
-        } else if (isU(R)) {
-            f = cur(R, 'a', false);
         } else if (isT(R)) {
             f = "(n == 1 ? " + lit(1.0) + " : " + lit(0.0) + ")";
         }
@@ -2416,6 +2435,7 @@ struct TeamGen {
             }
             o << "};\n";
         }
+        o << "static __device__ __forceinline__ hyk_real hyk_flip(hyk_real x, int neg) { return HYK_NEG_IF(x, neg); }\n";
         // (C: the team's cold rows, HYK_CROW(i, n) = C[n * HYK_NEQ + i]; unused without them)
         o << "#define HYK_CROW(i, n) C[(n) * HYK_NEQ + (i)]\n";
         o << "static __device__ __noinline__ void hyk_tjets(hyk_real *__restrict__ S, hyk_real *__restrict__ C, "
