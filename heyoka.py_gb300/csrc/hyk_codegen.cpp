@@ -1396,11 +1396,19 @@ struct Gen {
         }
     }
 
-    // The order-0 reciprocals the forward recurrences kept (split functions).
+    // The order-0 reciprocals the forward recurrences kept (split functions); the
+    // pinned arithmetic divides and keeps none.
     void emit_inverses() {
         for (uint32_t k = 0; k < d.n_ops; ++k) {
             const uint32_t u = N + k;
-            if (!alias[u] && islot[u] >= 0) o << "    const double " << inv0(u) << " = " << smem((uint32_t)islot[u]) << ";\n";
+            if (alias[u] || islot[u] < 0) continue;
+            const auto &op = d.ops[k];
+            std::string e = smem((uint32_t)islot[u]);
+            if (pin)
+                e = op.op == HYK_OP_DIV    ? "1.0 / " + val(res(op.b), 0)
+                    : op.op == HYK_OP_SQRT ? "1.0 / (2.0 * sqrt(" + val(res(op.a), 0) + "))"
+                                           : "1.0 / " + val(res(op.a), 0);
+            o << "    const double " << inv0(u) << " = " << e << ";\n";
         }
     }
 
@@ -2668,7 +2676,7 @@ bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, si
 // with the adjoint, the reverse sweep) for CPU checks of the generator: one
 // lane, HYK_BLK = 1, the CUDA intrinsics mapped to their host equivalents.
 bool generate_host(const Dec &d, uint32_t order, bool adjoint, std::string &src, std::string &err, bool team, bool f32,
-                   bool cold) {
+                   bool cold, bool pin) {
     PrecisionScope ps(f32);
     if (order < 2) {
         err = "the Taylor order must be at least 2";
@@ -2721,7 +2729,7 @@ bool generate_host(const Dec &d, uint32_t order, bool adjoint, std::string &src,
         src = h.str();
         return true;
     }
-    Gen g(d, order, false, adjoint);
+    Gen g(d, order, pin, adjoint);
     const double p = (double)order;
     std::ostringstream h;
     h << "#include <cmath>\n#include <cstdint>\n#define __device__\n#define __noinline__\n"
@@ -2730,7 +2738,7 @@ bool generate_host(const Dec &d, uint32_t order, bool adjoint, std::string &src,
              "static inline float __fmaf_rn(float a, float b, float c) { return std::fma(a, b, c); }\n"
          "static inline void __syncwarp() {}\n#define HYK_WARP_SYNC()\n";
     h << kDmath << "\n";
-    h << (f32 ? "typedef float hyk_real;\n" : "typedef double hyk_real;\n") << precision_header(false);
+    h << (f32 ? "typedef float hyk_real;\n" : "typedef double hyk_real;\n") << precision_header(pin);
     h << "#define HYK_NEQ " << d.n_eq << "\n#define HYK_NPARS " << d.n_pars << "\n#define HYK_ORDER " << order
       << "\n#define HYK_BLK 1\n#define HYK_STRIDE 1\n#define HYK_NSLOT " << g.nslot << "\n#define HYK_PAR_SLOT " << g.par_slot
       << "\n#define HYK_RHOFAC " << lit(rhofac_of(order)) << "\n#define HYK_INV_P " << lit(recip(p)) << "\n#define HYK_INV_PM1 "

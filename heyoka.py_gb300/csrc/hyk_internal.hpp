@@ -75,9 +75,10 @@ bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, si
 
 // Host (CPU) translation unit of the same recurrences, for checks of the
 // generator (team: the team form's recurrences, run by a team of one; cold:
-// with cold state rows where the system allows them).
+// with cold state rows where the system allows them; pin: the lane form's
+// recurrences and reverse sweep in the pinned arithmetic).
 bool generate_host(const Dec &d, uint32_t order, bool adjoint, std::string &src, std::string &err, bool team = false,
-                   bool f32 = false, bool cold = false);
+                   bool f32 = false, bool cold = false, bool pin = false);
 
 // The recurrences in the reference's arithmetic over an element type chosen
 // by the includer (a vector of lanes for the compiled CPU stepper).

@@ -1313,7 +1313,7 @@ int hyk_codegen_check(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     if (flops) *flops = g.flops;
     if (verbose == 3) {  // host translation unit (CPU checks of the generator)
         std::string hs;
-        if (!hyk::generate_host(d, order, adjoint, hs, err, false, f32)) return fail(HYK_ERR_INVALID, err);
+        if (!hyk::generate_host(d, order, adjoint, hs, err, false, f32, false, pin)) return fail(HYK_ERR_INVALID, err);
         if (log && log_len) std::snprintf(log, log_len, "%s", hs.c_str());
         return 0;
     }
