@@ -350,8 +350,9 @@ static uint32_t default_team(const hyk::TeamInfo &ti, size_t lane_bytes, size_t 
 // 41 s and 0.8 s).  The default form is kept unless another is estimated 5 %
 // faster, and of teams within 8 % of the fastest the one with the fewest
 // instructions is taken: the last trajectories then run fastest.
-static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool large, size_t real_bytes, const Device &dv,
-                               uint64_t n) {
+// (cold: with cold state rows where the system has them)
+static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool large, bool cold, size_t real_bytes,
+                               const Device &dv, uint64_t n) {
     const double smsp = 4.0 * dv.n_sm;
     auto cost = [&](double c, double warps, double resident) {
         const double w = 0.7 * warps / smsp, k = std::min(resident, w);
@@ -362,7 +363,7 @@ static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool larg
     c[0] = cost(large ? 4.0 : 1.15, (double)n / 32.0, 2.0);
     for (uint32_t l = 1; l <= 5; ++l) {
         const uint32_t T = 1u << l;
-        const size_t cta = (size_t)(32 / T) * ti.slots(T, ti.n_slot_cold != 0) * real_bytes;
+        const size_t cta = (size_t)(32 / T) * ti.slots(T, cold) * real_bytes;
         c[l] = INFINITY;
         if (cta > (size_t)dv.smem_optin) continue;
         const double resident = std::min(16.0, (double)((size_t)dv.smem_per_sm / (cta + 1024))) / 4.0;
@@ -731,12 +732,13 @@ int hyk_config_for(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t *c
     const size_t lane_bytes = (size_t)hyk::count_slots(d, order) * sizeof(double);
     const uint32_t dflt = default_team(ti, lane_bytes, sizeof(double), *dv);
     const bool large = (uint64_t)d.n_ops * order > 3000 || lane_bytes * 32 > (size_t)dv->smem_optin;
-    const uint32_t team = team_for_batch(ti, dflt, large, sizeof(double), *dv, n_lanes);
+    const bool cold = ti.n_slot_cold != 0 && !(c.flags & HYK_CFG_NO_COLD_ROWS);
+    const uint32_t team = team_for_batch(ti, dflt, large, cold, sizeof(double), *dv, n_lanes);
     if (team != dflt) c.team_size = team ? team : 1;
     // A team form whose trajectories are all resident at once without cold
     // state rows does without them (331 six-body members: teams of 32 87 us a
     // step with them, 76 without; teams of 16 124 and 99).
-    if (team && ti.n_slot_cold) {
+    if (team && cold) {
         const size_t cta = (size_t)(32 / team) * ti.slots(team, false) * sizeof(double);
         const uint64_t ctas = cta > (size_t)dv->smem_optin ? 0 : std::min<uint64_t>(24, (size_t)dv->smem_per_sm / (cta + 1024));
         if (n_lanes <= ctas * dv->n_sm * (32 / team)) c.flags |= HYK_CFG_NO_COLD_ROWS;
