@@ -2622,7 +2622,7 @@ bool team_layout(const Dec &d, uint32_t order, TeamInfo &info, std::string &err)
 }
 
 bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, size_t kparams_size, GenOut &out,
-                   std::string &err, bool high_acc, bool f32, bool gmem, bool cold) {
+                   std::string &err, bool high_acc, bool f32, bool gmem, bool cold, bool spread) {
     if (order < 2) {
         err = "the Taylor order must be at least 2";
         return false;
@@ -2638,7 +2638,7 @@ bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, si
         return false;
     }
     tg.g.emit_jets();  // flop count of the same recurrences
-    tg.spread_powers(team);
+    if (spread) tg.spread_powers(team);
     tg.plan_rounds(team);
     tg.full = TeamGen::is_full(d, order);
     const double p = (double)order;

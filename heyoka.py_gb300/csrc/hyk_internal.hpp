@@ -66,12 +66,15 @@ struct TeamInfo {
     uint32_t n_spread[6] = {0, 0, 0, 0, 0, 0};  // doubles more for the powers' products spread over the team
     uint32_t n_raw = 0, n_raw_cold = 0;         // n_slot and n_slot_cold before the padding to an odd number
     // Doubles per trajectory of a team of T threads (odd).
-    uint32_t slots(uint32_t T, bool cold) const { return ((cold ? n_raw_cold : n_raw) + n_spread[__builtin_ctz(T)]) | 1u; }
+    uint32_t slots(uint32_t T, bool cold, bool spread) const {
+        return ((cold ? n_raw_cold : n_raw) + (spread ? n_spread[__builtin_ctz(T)] : 0u)) | 1u;
+    }
 };
 // false (with the reason) when an operation has no team-form code.
 bool team_layout(const Dec &d, uint32_t order, TeamInfo &info, std::string &err);
 bool generate_team(const Dec &d, uint32_t order, uint32_t team, uint32_t tpb, size_t kparams_size, GenOut &out,
-                   std::string &err, bool high_acc = false, bool f32 = false, bool gmem = false, bool cold = false);
+                   std::string &err, bool high_acc = false, bool f32 = false, bool gmem = false, bool cold = false,
+                   bool spread = true);
 
 // Host (CPU) translation unit of the same recurrences, for checks of the
 // generator (team: the team form's recurrences, run by a team of one; cold:

@@ -329,6 +329,14 @@ static uint32_t default_team(const hyk::TeamInfo &ti, size_t lane_bytes, size_t 
     return team;
 }
 
+// Doubles per trajectory of a team of T threads, tpc trajectories to a CTA:
+// with the powers' products spread over the team where they fit the shared
+// memory beside the coefficients.
+static uint32_t team_slots(const hyk::TeamInfo &ti, uint32_t T, bool cold, size_t tpc, size_t real_bytes, const Device &dv) {
+    const uint32_t s = ti.slots(T, cold, true);
+    return tpc * s * real_bytes <= (size_t)dv.smem_optin ? s : ti.slots(T, cold, false);
+}
+
 // The form for a batch of n trajectories (hyk_config_for), by an estimate of
 // the time of one step of all of them in units of a lane-form step's FP64
 // instructions, 64 cycles each whatever the active lanes of the warp.
@@ -363,7 +371,7 @@ static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool larg
     c[0] = cost(large ? 4.0 : 1.15, (double)n / 32.0, 2.0);
     for (uint32_t l = 1; l <= 5; ++l) {
         const uint32_t T = 1u << l;
-        const size_t cta = (size_t)(32 / T) * ti.slots(T, cold) * real_bytes;
+        const size_t cta = (size_t)(32 / T) * team_slots(ti, T, cold, 32 / T, real_bytes, dv) * real_bytes;
         c[l] = INFINITY;
         if (cta > (size_t)dv.smem_optin) continue;
         const double resident = std::min(16.0, (double)((size_t)dv.smem_per_sm / (cta + 1024))) / 4.0;
@@ -452,7 +460,8 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     }
     if (m->team) {
         if (blk == 0) blk = 32;
-        nslot = ti.slots(m->team, false);
+        nslot = (m->cfg.flags & HYK_CFG_GLOBAL_JETS) ? ti.slots(m->team, false, true)
+                                                     : team_slots(ti, m->team, false, blk / m->team, real_bytes, dv);
         lane_bytes = (size_t)nslot * real_bytes;
     }
     // Lane form of a system whose coefficients do not fit 32 lanes of shared
@@ -482,11 +491,12 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
         // trajectories instead of six).
         if (!m->gmem && ti.n_slot_cold && !(m->cfg.flags & HYK_CFG_NO_COLD_ROWS)) {
             const size_t tpc = blk / m->team;
-            const size_t hot = tpc * ti.slots(m->team, false) * real_bytes, cold = tpc * ti.slots(m->team, true) * real_bytes;
+            const uint32_t cslots = team_slots(ti, m->team, true, tpc, real_bytes, dv);
+            const size_t hot = tpc * lane_bytes, cold = tpc * cslots * real_bytes;
             const uint32_t ch = hot > (size_t)dv.smem_optin ? 0 : (uint32_t)((size_t)dv.smem_per_sm / (hot + 1024));
             const uint32_t cc = cold > (size_t)dv.smem_optin ? 0 : (uint32_t)((size_t)dv.smem_per_sm / (cold + 1024));
             if (std::min<uint32_t>(cc, 32) > std::min<uint32_t>(ch, 32)) {
-                nslot = ti.slots(m->team, true);
+                nslot = cslots;
                 lane_bytes = (size_t)nslot * real_bytes;
                 m->ncold = m->d.n_eq;
                 m->cold_ctas = (int)std::min<uint32_t>(cc, 32);
@@ -585,7 +595,8 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     hyk::GenOut g;
     const bool high_acc = (m->cfg.flags & HYK_CFG_HIGH_ACCURACY) != 0;
     if (m->team) {
-        if (!hyk::generate_team(m->d, order, m->team, blk, sizeof(KParams), g, err, high_acc, f32, m->gmem, m->ncold != 0))
+        if (!hyk::generate_team(m->d, order, m->team, blk, sizeof(KParams), g, err, high_acc, f32, m->gmem, m->ncold != 0,
+                                nslot == ti.slots(m->team, m->ncold != 0, true)))
             return fail(HYK_ERR_INVALID, err);
     } else if (!hyk::generate(m->d, order, pin, blk, sizeof(KParams), g, err, adjoint, m->gmem ? m->gmem_threads : 0,
                               high_acc, f32, m->ncold ? m->cold_threads : 0, m->gmem, inreg, min_ctas)) {
@@ -739,7 +750,7 @@ int hyk_config_for(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t *c
     // state rows does without them (331 six-body members: teams of 32 87 us a
     // step with them, 76 without; teams of 16 124 and 99).
     if (team && cold) {
-        const size_t cta = (size_t)(32 / team) * ti.slots(team, false) * sizeof(double);
+        const size_t cta = (size_t)(32 / team) * team_slots(ti, team, false, 32 / team, sizeof(double), *dv) * sizeof(double);
         const uint64_t ctas = cta > (size_t)dv->smem_optin ? 0 : std::min<uint64_t>(24, (size_t)dv->smem_per_sm / (cta + 1024));
         if (n_lanes <= ctas * dv->n_sm * (32 / team)) c.flags |= HYK_CFG_NO_COLD_ROWS;
     }
