@@ -337,6 +337,37 @@ static uint32_t team_slots(const hyk::TeamInfo &ti, uint32_t T, bool cold, size_
     return tpc * s * real_bytes <= (size_t)dv.smem_optin ? s : ti.slots(T, cold, false);
 }
 
+// Lane form of a small system: the histories in registers, and the state
+// rows up to the state update.  A term of a convolution then needs no
+// shared-memory loads, which bound the float kernels and lengthened the step of
+// a warp alone on its FP64 unit.  2^20 Kepler orbits in float (order 9),
+// propagation kernel alone: 3.85 ms with the histories in shared memory (two
+// CTAs of 256), 2.86 with them in registers, 2.41 with the rows too, in ten
+// CTAs of 64 and 96 registers a thread (six of 128 and 80 registers 2.66, five
+// of 128 2.54).  Pendulum (order 20): 26, 24 and 22 us a step.
+struct RegForm {
+    bool on = false;
+    uint32_t nslot = 0, blk = 0, min_ctas = 0;
+};
+static RegForm register_form(const hyk::Dec &d, uint32_t order, uint32_t flags, uint32_t blk, uint64_t smem_per_sm) {
+    RegForm r;
+    const bool f32 = (flags & HYK_CFG_FLOAT32) != 0;
+    const uint32_t n_live = (flags & (HYK_CFG_PIN_ARITH | HYK_CFG_ADJOINT | HYK_CFG_GLOBAL_JETS)) ? 0 : hyk::register_values(d, order, f32);
+    if (!n_live) return r;
+    r.on = true;
+    r.blk = blk;
+    r.nslot = hyk::count_slots(d, order, false, false, false, nullptr, false, true);
+    if (f32 && blk == 0) {
+        // about 50 registers besides the histories (the rows of the other
+        // state variables among them); at most 768 threads an SM
+        r.blk = 64;
+        const uint32_t regs = (n_live + 50 + 7) / 8 * 8;
+        r.min_ctas = std::min<uint32_t>(768, 65536 / regs) / r.blk;
+        r.min_ctas = std::min<uint32_t>(r.min_ctas, (uint32_t)(smem_per_sm / (r.blk * (size_t)r.nslot * sizeof(float) + 1024)));
+    }
+    return r;
+}
+
 // The form for a batch of n trajectories (hyk_config_for), by an estimate of
 // the time of one step of all of them in units of a lane-form step's FP64
 // instructions, 64 cycles each whatever the active lanes of the warp.
@@ -433,30 +464,12 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     } else if (want_team == 0 && team_ok) {
         m->team = default_team(ti, lane_bytes, real_bytes, dv);
     }
-    // Lane form of a small system: the histories in registers, and the state
-    // rows up to the state update.  A term of a convolution then needs no
-    // shared-memory loads, which bound the float kernels and lengthened the step of
-    // a warp alone on its FP64 unit.  2^20 Kepler orbits in float (order 9),
-    // propagation kernel alone: 3.85 ms with the histories in shared memory (two
-    // CTAs of 256), 2.86 with them in registers, 2.41 with the rows too, in ten
-    // CTAs of 64 and 96 registers a thread (six of 128 and 80 registers 2.66, five
-    // of 128 2.54).  Pendulum (order 20): 26, 24 and 22 us a step.
-    const uint32_t n_live = !m->team && !pin && !adjoint && !(m->cfg.flags & HYK_CFG_GLOBAL_JETS)
-                                ? hyk::register_values(m->d, order, f32)
-                                : 0;
-    const bool inreg = n_live != 0;
-    uint32_t min_ctas = 0;
+    const RegForm reg = m->team ? RegForm{} : register_form(m->d, order, m->cfg.flags, blk, dv.smem_per_sm);
+    const bool inreg = reg.on;
     if (inreg) {
-        nslot = hyk::count_slots(m->d, order, false, false, false, nullptr, false, true);
+        nslot = reg.nslot;
         lane_bytes = (size_t)nslot * real_bytes;
-        if (f32 && blk == 0) {
-            // about 50 registers besides the histories (the rows of the other
-            // state variables among them); at most 768 threads an SM
-            blk = 64;
-            const uint32_t regs = (n_live + 50 + 7) / 8 * 8;
-            min_ctas = std::min<uint32_t>(768, 65536 / regs) / blk;
-            min_ctas = std::min<uint32_t>(min_ctas, (uint32_t)((size_t)dv.smem_per_sm / (blk * lane_bytes + 1024)));
-        }
+        blk = reg.blk;
     }
     if (m->team) {
         if (blk == 0) blk = 32;
@@ -599,7 +612,7 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
                                 nslot == ti.slots(m->team, m->ncold != 0, true)))
             return fail(HYK_ERR_INVALID, err);
     } else if (!hyk::generate(m->d, order, pin, blk, sizeof(KParams), g, err, adjoint, m->gmem ? m->gmem_threads : 0,
-                              high_acc, f32, m->ncold ? m->cold_threads : 0, m->gmem, inreg, min_ctas)) {
+                              high_acc, f32, m->ncold ? m->cold_threads : 0, m->gmem, inreg, reg.min_ctas)) {
         return fail(HYK_ERR_INVALID, err);
     }
     if (g.n_slot != nslot || g.n_cold != m->ncold) return fail(HYK_ERR_INVALID, "internal: slot count mismatch");
@@ -1300,7 +1313,10 @@ int hyk_codegen_check(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
         if (log && log_len) std::snprintf(log, log_len, "%s", hs.c_str());
         return 0;
     }
-    const uint32_t slots = hyk::count_slots(d, order, adjoint, pin);
+    // (with the histories in registers where the runtime keeps them there)
+    RegForm reg;
+    if (team <= 1) reg = register_form(d, order, cfg ? cfg->flags : 0u, cfg ? cfg->block_lanes : 0u, 228u * 1024);
+    const uint32_t slots = reg.on ? reg.nslot : hyk::count_slots(d, order, adjoint, pin);
     // The global-memory layout when 32 lanes do not fit shared memory or on
     // request (HYK_CFG_GLOBAL_JETS), with the slot stride of two CTAs per SM.
     const bool want_g = (uint64_t)slots * (f32 ? 4 : 8) * 32 > 227u * 1024 || (cfg && (cfg->flags & HYK_CFG_GLOBAL_JETS));
@@ -1308,7 +1324,7 @@ int hyk_codegen_check(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     // The cold-state-row layout (as the runtime may pick it), with the rows
     // sized for one CTA per SM of a 152-SM GPU.
     uint32_t ncold = 0;
-    if (!gstride && !adjoint && d.ev.empty() && !(cfg && (cfg->flags & HYK_CFG_NO_COLD_ROWS)))
+    if (!reg.on && !gstride && !adjoint && d.ev.empty() && !(cfg && (cfg->flags & HYK_CFG_NO_COLD_ROWS)))
         hyk::count_slots(d, order, adjoint, pin, true, &ncold);
     const uint64_t cstride = ncold ? 152ull * blk : 0;
     hyk::GenOut g;
@@ -1318,8 +1334,8 @@ int hyk_codegen_check(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
         if (!hyk::generate_team(d, order, team, cfg->block_lanes ? cfg->block_lanes : (tg ? 128 : 32), sizeof(KParams),
                                 g, err, high_acc, f32, tg, !(cfg->flags & HYK_CFG_NO_COLD_ROWS)))
             return fail(HYK_ERR_UNSUPPORTED, err);
-    } else if (!hyk::generate(d, order, pin, blk, sizeof(KParams), g, err, adjoint, gstride, high_acc, f32, cstride,
-                              gstride != 0)) {
+    } else if (!hyk::generate(d, order, pin, reg.on && reg.blk && !gstride ? reg.blk : blk, sizeof(KParams), g, err, adjoint,
+                              gstride, high_acc, f32, cstride, gstride != 0, reg.on, reg.min_ctas)) {
         return fail(HYK_ERR_INVALID, err);
     }
     if (n_slot) *n_slot = g.n_slot;

@@ -479,7 +479,8 @@ int hyk_fp64_peak(int device, double millis, double *flops_per_s);
 int hyk_fp32_peak(int device, double millis, double *flops_per_s);
 
 /* Build check without a GPU: generate the module source for `d` at `order`
- * (block size cfg->block_lanes, default 128; the lane form with cold state
+ * (block size cfg->block_lanes, default 128; the lane form with the histories
+ * in registers where hyk_module_create keeps them there, else with cold state
  * rows unless cfg->flags has HYK_CFG_NO_COLD_ROWS) and compile it with NVRTC
  * for sm_103a.  `log` receives the NVRTC log (ptxas register and spill
  * statistics when `verbose` is 1; the generated source, without compiling,
