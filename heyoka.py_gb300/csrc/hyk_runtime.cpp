@@ -345,6 +345,18 @@ static uint32_t team_slots(const hyk::TeamInfo &ti, uint32_t T, bool cold, size_
 // CTAs of 256), 2.86 with them in registers, 2.41 with the rows too, in ten
 // CTAs of 64 and 96 registers a thread (six of 128 and 80 registers 2.66, five
 // of 128 2.54).  Pendulum (order 20): 26, 24 and 22 us a step.
+//
+// The shared memory then holds all the state rows (for outputs), while cold rows
+// (below) would take one slot a variable.  In double precision, where the
+// recurrences of linear systems leave little to gain, it needs room for five warps on an
+// SM.  200000 lanes, registers against cold rows: 8 linear equations (five warps) 3.81
+// and 3.87 ms (chain), 4.32 and 4.39 (oscillators), 9 and 10 equations (four
+// warps) 2.30 and 2.06, 2.56 and 2.24, 5.25 and 4.63; a pendulum or Lorenz system with
+// up to five integrals (seven and eight equations) 27.3 and 28.1, 84.5 and 90.3.  That the
+// rows of linear systems spill some registers (three oscillators 312 B, 2.82
+// and 3.03 ms) costs less than the loads.  Float systems gain at every size that
+// does not go to global memory (2^20 lanes, 12, 24 and 44 equations 0.65 and 1.49, 1.65
+// and 4.37, 4.00 and 6.77 ms).
 struct RegForm {
     bool on = false;
     uint32_t nslot = 0, blk = 0, min_ctas = 0;
@@ -354,9 +366,12 @@ static RegForm register_form(const hyk::Dec &d, uint32_t order, uint32_t flags, 
     const bool f32 = (flags & HYK_CFG_FLOAT32) != 0;
     const uint32_t n_live = (flags & (HYK_CFG_PIN_ARITH | HYK_CFG_ADJOINT | HYK_CFG_GLOBAL_JETS)) ? 0 : hyk::register_values(d, order, f32);
     if (!n_live) return r;
+    r.nslot = hyk::count_slots(d, order, false, false, false, nullptr, false, true);
+    uint32_t ncold = 0;
+    if (!f32 && d.ev.empty() && !(flags & HYK_CFG_NO_COLD_ROWS)) hyk::count_slots(d, order, false, false, true, &ncold);
+    if (ncold && smem_per_sm / (32 * (size_t)r.nslot * sizeof(double) + 1024) < 5) return r;
     r.on = true;
     r.blk = blk;
-    r.nslot = hyk::count_slots(d, order, false, false, false, nullptr, false, true);
     if (f32 && blk == 0) {
         // about 50 registers besides the histories (the rows of the other
         // state variables among them); at most 768 threads an SM

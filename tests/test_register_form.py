@@ -3,6 +3,7 @@ the source that hyk_codegen_check generates for the GPU, which compiles."""
 
 import ctypes
 
+import numpy as np
 import pytest
 
 import hyk
@@ -32,3 +33,33 @@ def test_the_check_follows_the_module(libhyk, flags, inreg):
     if flags & _lib.HYK_CFG_FLOAT32:
         assert "#define HYK_TPB 64\n" in src and "__launch_bounds__(HYK_TPB, " in src
     _source(libhyk, W.pendulum_sys(), 20, flags, compile_it=True)
+
+
+def linear(n):
+    x = hyk.make_vars(*["x{}".format(i) for i in range(n)])
+    return [(x[i], -x[(i + 1) % n]) for i in range(n)]
+
+
+@pytest.mark.parametrize("n,flags,inreg", [
+    (2, 0, 1), (8, 0, 1),  # five warps' rows in the shared memory of an SM
+    (9, 0, 0), (10, 0, 0), (9, _lib.HYK_CFG_NO_COLD_ROWS, 1),
+    (24, _lib.HYK_CFG_FLOAT32, 1)])
+def test_rows_that_leave_too_few_warps(libhyk, n, flags, inreg):
+    src, ns = _source(libhyk, linear(n), 9 if flags & _lib.HYK_CFG_FLOAT32 else 20, flags)
+    assert "#define HYK_INREG {}\n".format(inreg) in src
+    assert ns == (n * (10 if flags & _lib.HYK_CFG_FLOAT32 else 21) if inreg else n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["persistent", "plain"])
+@pytest.mark.parametrize("n", [1, 8, 9, 10])
+def test_linear_systems_bitwise(oracle, n, mode):
+    sys_ = linear(n) if n > 1 else [(hyk.make_vars("x"), hyk.par[0] * hyk.make_vars("x"))]
+    st = np.random.default_rng(n).uniform(0.5, 1.0, (n, 333))
+    pars = np.random.default_rng(7).uniform(-1.0, -0.5, (1, 333)) if n == 1 else None
+    ta = hyk.taylor_adaptive_batch(sys_, st, pars=pars, team_size=1, prop_mode=mode)
+    tf = np.linspace(0.5, 9.0, 333)
+    ta.propagate_until(tf)
+    o = oracle.Oracle(sys_, st, pars=pars, order=ta.order, mode=1)
+    o.propagate_until(tf)
+    assert np.array_equal(np.asarray(ta.state), o.state)
