@@ -536,6 +536,7 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
         // own slots for the order-0 reciprocals.
         nslot = hyk::count_slots(m->d, order, adjoint, pin, false, nullptr, true);
         lane_bytes = (size_t)nslot * real_bytes;
+        blk = m->cfg.block_lanes;  // (not the register form's)
         // Two CTAs of 128 threads per SM by default: at most 255 registers a
         // thread, so both fit the register file, and eight warps hide the
         // latency of the global-memory coefficients better than four.

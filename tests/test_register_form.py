@@ -63,3 +63,34 @@ def test_linear_systems_bitwise(oracle, n, mode):
     o = oracle.Oracle(sys_, st, pars=pars, order=ta.order, mode=1)
     o.propagate_until(tf)
     assert np.array_equal(np.asarray(ta.state), o.state)
+
+
+@pytest.mark.gpu
+def test_block_size_of_a_float_system_in_global_memory(oracle):
+    """Short histories, but rows that leave room for fewer than four warps."""
+    sys_ = linear(60)
+    st = np.random.default_rng(4).uniform(0.5, 1.0, (60, 200)).astype(np.float32)
+    ta = hyk.taylor_adaptive_batch(sys_, st, team_size=1, fp_type=np.float32)
+    assert ta.module_info["smem_per_lane"] == 0 and ta.module_info["block_lanes"] == 128
+    ta.propagate_until(3.0)
+    o = oracle.Oracle(sys_, st.astype(np.float64), order=ta.order, mode=1, prec=2)
+    o.propagate_until(3.0)
+    assert np.array_equal(np.asarray(ta.state).astype(np.float64), o.state)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fp", [np.float64, np.float32])
+@pytest.mark.parametrize("name", ["pendulum", "linear"])
+def test_coefficients_copied_from_registers(oracle, name, fp):
+    """A step's coefficients, which outputs read from the shared memory."""
+    sys_ = W.pendulum_sys() if name == "pendulum" else linear(4)
+    st = np.random.default_rng(6).uniform(0.1, 1.0, (len(sys_), 99)).astype(fp)
+    f32 = fp == np.float32
+    ta = hyk.taylor_adaptive_batch(sys_, st, team_size=1, fp_type=np.float32 if f32 else float)
+    ta.propagate_until(0.7)
+    ta.step(write_tc=True)
+    o = oracle.Oracle(sys_, st.astype(np.float64), order=ta.order, mode=1, prec=2 if f32 else 0)
+    o.propagate_until(0.7)
+    o.step()
+    assert np.array_equal(np.asarray(ta.state).astype(np.float64), o.state)
+    assert np.array_equal(np.asarray(ta.tc).astype(np.float64), o.tc)
