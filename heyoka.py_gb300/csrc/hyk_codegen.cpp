@@ -369,6 +369,7 @@ struct Gen {
                 cst[u] = kconst(op.a) && kconst(op.b);
             }
         }
+        time_degrees();
         if (!pin) {
             fz = hyk_fuse_plan(N, d.n_ops, d.ops.data(), d.rhs.data(), (uint32_t)d.ev.size(), d.ev.data());
             for (uint32_t k = 0; k < d.n_ops; ++k)
@@ -376,6 +377,36 @@ struct Gen {
         }
         analyse();
     }
+
+    // Degree in time of each u-variable that is a polynomial in it (a state variable
+    // whose right-hand side is one among them), -1 of the others.
+    std::vector<int> deg;
+    void time_degrees() {
+        deg.assign(NU, -1);
+        auto of = [&](const hyk_arg_t &a) { return a.kind == HYK_ARG_U ? deg[a.idx] : a.kind == HYK_ARG_TIME ? 1 : 0; };
+        for (bool more = true; more;) {
+            for (uint32_t k = 0; k < d.n_ops; ++k) {
+                const auto &op = d.ops[k];
+                const int a = of(op.a), b = of(op.b);
+                int r = -1;
+                if (a >= 0 && b >= 0) {
+                    if (op.op == HYK_OP_ADD || op.op == HYK_OP_SUB || op.op == HYK_OP_NEG) r = std::max(a, b);
+                    else if (op.op == HYK_OP_MUL) r = a + b;
+                    else if (op.op == HYK_OP_SQUARE) r = 2 * a;
+                    else if (b == 0 && (op.op == HYK_OP_DIV || a == 0)) r = a;
+                }
+                deg[N + k] = std::min(r, 1 << 20);
+            }
+            more = false;
+            for (uint32_t i = 0; i < N; ++i)
+                if (deg[i] < 0 && of(d.rhs[i]) >= 0) {
+                    deg[i] = of(d.rhs[i]) + 1;
+                    more = true;
+                }
+        }
+    }
+    // Whether a base's coefficients vanish at orders that a power reads.
+    bool vanishes(const Ref &r) const { return r.kind == HYK_ARG_U && deg[r.u] >= 0 && deg[r.u] + 2 < (int)p; }
 
     Ref res(const hyk_arg_t &a) const {
         Ref r;
@@ -845,7 +876,8 @@ struct Gen {
             // 1656 FP64 instructions of a step, propagation kernel 247.0 ->
             // 227.4 ms.  Not where the recurrences are split into functions: the
             // CR3BP kernel there waits for its instructions, and the longer code
-            // took 20011 trajectories from 8.55 to 9.68 ms.
+            // took 20011 trajectories from 8.55 to 9.68 ms.  Nor for a base that is a
+            // polynomial in time, whose higher orders are zero and out of that range.
             const std::string bad = "bad" + std::to_string(u) + "_" + std::to_string(n);
             auto chain = [&](const std::string &name, const std::string &pre, bool ints) {
                 Acc s{name};
@@ -865,7 +897,7 @@ struct Gen {
                 }
                 return s;
             };
-            const bool ints = fmaops() && !split && n > 1 && kpack(powcoef(n, 1, alpha)) != 0;
+            const bool ints = fmaops() && !split && !vanishes(A) && n > 1 && kpack(powcoef(n, 1, alpha)) != 0;
             if (ints) o << "    unsigned " << bad << " = 0;\n";
             Acc s = chain(acc, "t", ints);
             if (ints) {
@@ -2290,7 +2322,8 @@ struct TeamGen {
                 out(u, false, "HYK_MUL(HYK_MUL(acc, hyk_invn[n]), S[D.inv])");
                 break;
             }
-            const bool ints = int_coefs(op.b.num);
+            bool ints = int_coefs(op.b.num);
+            for (uint32_t m : gr.members) ints = ints && !g.vanishes(g.res(d.ops[m - N].a));
             o << "            hyk_real acc;\n";
             if (ints) o << "            unsigned bad = 0;\n";
             chain(ints);
