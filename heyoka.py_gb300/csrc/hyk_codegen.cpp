@@ -2587,7 +2587,7 @@ bool generate(const Dec &d, uint32_t order, bool pin_arith, uint32_t blk, size_t
         h << "#define HYK_FMA_ACC(a, b, c) HYK_FMA((a), (b), (c))\n";
         h << rho_macro();
     }
-    h << "#define HYK_LB __launch_bounds__(HYK_TPB" << (g.inreg && min_ctas ? ", " + std::to_string(min_ctas) : "") << ")\n";
+    h << "#define HYK_LB __launch_bounds__(HYK_TPB" << (min_ctas ? ", " + std::to_string(min_ctas) : "") << ")\n";
     h << "#define HYK_INREG " << (g.inreg ? 1 : 0) << "\n";
     h << "#define HYK_PHASE " << (!g_f32 && !g.inreg && d.ev.empty() ? 1 : 0) << "\n";
     if (adjoint) h << "#define HYK_ADJOINT 1\n";

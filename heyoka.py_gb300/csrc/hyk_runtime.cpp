@@ -274,6 +274,7 @@ struct hyk_module {
     int adj_ctas_per_sm = 0;
     uint32_t team = 0;           // threads per trajectory (team form); 0 = lane form
     bool f32 = false;            // single precision
+    bool inreg = false;          // histories in registers (lane form of small systems)
     bool gmem = false;           // Taylor coefficients in a global buffer (large systems)
     uint64_t gmem_threads = 0;   // threads of the fixed grid in that mode
     uint32_t ncold = 0;          // cold state rows in the global buffer (0: none)
@@ -621,53 +622,83 @@ int hyk_module_create(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t
     if (m->smem > (size_t)dv.smem_optin)
         return fail(HYK_ERR_UNSUPPORTED, "shared memory per CTA (" + std::to_string(m->smem) + ") exceeds the device limit");
 
-    hyk::GenOut g;
-    const bool high_acc = (m->cfg.flags & HYK_CFG_HIGH_ACCURACY) != 0;
-    if (m->team) {
-        if (!hyk::generate_team(m->d, order, m->team, blk, sizeof(KParams), g, err, high_acc, f32, m->gmem, m->ncold != 0,
-                                nslot == ti.slots(m->team, m->ncold != 0, true)))
-            return fail(HYK_ERR_INVALID, err);
-    } else if (!hyk::generate(m->d, order, pin, blk, sizeof(KParams), g, err, adjoint, m->gmem ? m->gmem_threads : 0,
-                              high_acc, f32, m->ncold ? m->cold_threads : 0, m->gmem, inreg, reg.min_ctas)) {
-        return fail(HYK_ERR_INVALID, err);
-    }
-    if (g.n_slot != nslot || g.n_cold != m->ncold) return fail(HYK_ERR_INVALID, "internal: slot count mismatch");
-    m->src = (m->cfg.flags & HYK_CFG_DEBUG) ? "#define HYK_DEBUG 1\n" + g.src : g.src;
-    m->flops = g.flops;
-
-    const auto t0 = std::chrono::steady_clock::now();
-    const std::string key = std::to_string(fnv1a(m->src)) + "_sm103a";
+    // Generates and compiles the module's source (min_ctas: the lane kernels'
+    // register bound, 0: none), from the caches when it was compiled before.
     std::string cubin;
-    {
-        std::lock_guard<std::mutex> lk(g_mtx);
-        auto it = g_cubin_cache.find(key);
-        if (it != g_cubin_cache.end()) cubin = it->second;
-    }
-    const std::string dpath = cache_dir() + "/" + key + ".cubin";
-    if (cubin.empty() && !std::getenv("HYK_NO_DISK_CACHE")) {
-        std::ifstream f(dpath, std::ios::binary);
-        if (f) {
-            std::ostringstream ss;
-            ss << f.rdbuf();
-            cubin = ss.str();
+    const auto t0 = std::chrono::steady_clock::now();
+    auto build = [&](uint32_t min_ctas) -> int {
+        hyk::GenOut g;
+        const bool high_acc = (m->cfg.flags & HYK_CFG_HIGH_ACCURACY) != 0;
+        if (m->team) {
+            if (!hyk::generate_team(m->d, order, m->team, blk, sizeof(KParams), g, err, high_acc, f32, m->gmem, m->ncold != 0,
+                                    nslot == ti.slots(m->team, m->ncold != 0, true)))
+                return fail(HYK_ERR_INVALID, err);
+        } else if (!hyk::generate(m->d, order, pin, blk, sizeof(KParams), g, err, adjoint, m->gmem ? m->gmem_threads : 0,
+                                  high_acc, f32, m->ncold ? m->cold_threads : 0, m->gmem, inreg, min_ctas)) {
+            return fail(HYK_ERR_INVALID, err);
         }
-    }
-    if (cubin.empty()) {
-        rc = compile_nvrtc(m->src, "hyk_module.cu", cubin, m->log);
-        if (rc) return rc;
-        if (!std::getenv("HYK_NO_DISK_CACHE")) {
-            std::string cmd = "mkdir -p '" + cache_dir() + "'";
-            if (std::system(cmd.c_str()) == 0) {
-                std::ofstream f(dpath + ".tmp", std::ios::binary);
-                f.write(cubin.data(), (std::streamsize)cubin.size());
-                f.close();
-                std::rename((dpath + ".tmp").c_str(), dpath.c_str());
+        if (g.n_slot != nslot || g.n_cold != m->ncold) return fail(HYK_ERR_INVALID, "internal: slot count mismatch");
+        m->src = (m->cfg.flags & HYK_CFG_DEBUG) ? "#define HYK_DEBUG 1\n" + g.src : g.src;
+        m->flops = g.flops;
+
+        const std::string key = std::to_string(fnv1a(m->src)) + "_sm103a";
+        cubin.clear();
+        {
+            std::lock_guard<std::mutex> lk(g_mtx);
+            auto it = g_cubin_cache.find(key);
+            if (it != g_cubin_cache.end()) cubin = it->second;
+        }
+        const std::string dpath = cache_dir() + "/" + key + ".cubin";
+        if (cubin.empty() && !std::getenv("HYK_NO_DISK_CACHE")) {
+            std::ifstream f(dpath, std::ios::binary);
+            if (f) {
+                std::ostringstream ss;
+                ss << f.rdbuf();
+                cubin = ss.str();
             }
         }
-    }
-    {
+        if (cubin.empty()) {
+            const int crc = compile_nvrtc(m->src, "hyk_module.cu", cubin, m->log);
+            if (crc) return crc;
+            if (!std::getenv("HYK_NO_DISK_CACHE")) {
+                std::string cmd = "mkdir -p '" + cache_dir() + "'";
+                if (std::system(cmd.c_str()) == 0) {
+                    std::ofstream f(dpath + ".tmp", std::ios::binary);
+                    f.write(cubin.data(), (std::streamsize)cubin.size());
+                    f.close();
+                    std::rename((dpath + ".tmp").c_str(), dpath.c_str());
+                }
+            }
+        }
         std::lock_guard<std::mutex> lk(g_mtx);
         g_cubin_cache[key] = cubin;
+        return 0;
+    };
+    m->inreg = inreg && !m->gmem;
+    rc = build(m->inreg ? reg.min_ctas : 0);
+    if (rc) return rc;
+    // Float lane form in shared memory: ptxas bounds its registers by the block
+    // size alone, and a few too many cost an SM a whole CTA.  Where up to
+    // 30 % fewer let in all the CTAs that the shared memory holds, they are
+    // asked for: 400000 lanes of six equations with elementary functions (211
+    // registers, 168 let in the second CTA of 192) 1.55 -> 1.18 ms, of a
+    // Lotka-Volterra chain (139, 128) 0.228 -> 0.165.  Not where the kernel needs far
+    // more: three bodies (255, 168), 400000 lanes 0.91 -> 0.74, but 1000 lanes
+    // 0.084 -> 0.117 with the spills.
+    if (f32 && !m->team && !m->gmem && !m->inreg) {
+        const uint32_t fit = std::min<uint32_t>((uint32_t)((size_t)dv.smem_per_sm / (m->smem + 1024)), 768u / blk);
+        CUmodule probe = nullptr;
+        CUfunction f = nullptr;
+        int regs = 0;
+        HYK_CU(drv().cuModuleLoadData(&probe, cubin.data()));
+        const bool known = drv().cuModuleGetFunction(&f, probe, "hyk_prop_kernel") == CUDA_SUCCESS &&
+                           drv().cuFuncGetAttribute(&regs, CU_FUNC_ATTRIBUTE_NUM_REGS, f) == CUDA_SUCCESS;
+        HYK_CU(drv().cuModuleUnload(probe));
+        const uint32_t need = (uint32_t)(regs + 7) / 8 * 8 * blk * fit;  // of the 65536 of an SM
+        if (known && fit >= 2 && need > 65536 && need <= 85000) {
+            rc = build(fit);
+            if (rc) return rc;
+        }
     }
     m->compile_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
 
