@@ -893,6 +893,13 @@ static void fill_lanes(KParams &k, const hyk_lanes_t *l) {
 // the speed of both (its FP64 unit is busy 78 % of the time with one warp).
 // A team's recurrences leave the unit idle half of the time with one warp,
 // and float lanes do not use it, so both take more warps at once.
+//
+// Float lanes outside the register form fill their warps: their code is long and
+// their coefficients are in memory, and few full warps, one on an SM before a
+// second, fetch both less often than many thin ones (1000 and 5000 lanes, thin and
+// full: four bodies 0.21 and 0.11, 0.21 and 0.12 ms, twelve equations with elementary functions
+// 0.42 and 0.33, 0.46 and 0.34; six equations 0.165 and 0.172 the other way, as
+// is the register form: Kepler 0.139 and 0.155).
 static uint64_t place(const hyk_module *m, uint64_t n, int ctas_per_sm, KParams &k) {
     const uint64_t sms = (uint64_t)m->dv->n_sm, wpc = m->blk / 32;
     const uint64_t units = m->team ? 32 / m->team : 32;
@@ -901,7 +908,7 @@ static uint64_t place(const hyk_module *m, uint64_t n, int ctas_per_sm, KParams 
     uint64_t layers = all, per = units;
     if (n <= room) {
         layers = base;
-        per = std::max<uint64_t>(1, (n + base * sms - 1) / (base * sms));
+        if (m->team || !m->f32 || m->inreg) per = std::max<uint64_t>(1, (n + base * sms - 1) / (base * sms));
     } else if (!m->team && !m->f32 && n <= room + room / 4) {
         layers = base;
     }
