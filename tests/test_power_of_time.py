@@ -56,3 +56,11 @@ def test_bitwise(oracle, name, team):
     o = oracle.Oracle(sys_, st, pars=pars, order=ta.order, mode=1)
     o.propagate_until(0.4)
     assert np.array_equal(np.asarray(ta.state), o.state)
+
+
+@pytest.mark.gpu
+def test_small_batch_of_powers_of_time_stays_in_the_lane_form():
+    x, y = hyk.make_vars("x", "y")
+    sys_ = [(x, (1.0 + hyk.time) ** -1.5 * y), (y, -x * (2.0 + hyk.time) ** -0.5)]
+    ta = hyk.taylor_adaptive_batch(sys_, np.ones((2, 1000)))
+    assert ta.module_info["team_size"] == 1
