@@ -86,6 +86,11 @@ def _propagate_taped(mod, x, pars, t0, tf, cap=None):
             nx[:cap], nt[:cap], nh[:cap] = ck_x, ck_t, ck_h
             ck_x, ck_t, ck_h, cap = nx, nt, nh, ncap
             a["status"] &= ~(_lib.LANE_CAPACITY | _lib.LANE_STOPPED)
+    # Until the backward pass only the rows that the longest lane filled stay
+    # (a copy: a view would keep the whole tape).
+    n = max(1, int(a["n_iter"].max()) if B else 0)
+    if n < cap:
+        ck_x, ck_t, ck_h = ck_x[:n].clone(), ck_t[:n].clone(), ck_h[:n].clone()
     return x, th, a, ck_x, ck_t, ck_h
 
 
