@@ -308,7 +308,8 @@ typedef struct hyk_prop {
      * its group's word stops before its next one (HYK_LANE_STOPPED, its
      * outcome that of its last step).  The one-launch-per-step form steps the
      * unfinished lanes in lockstep, so one call gives the reference's result;
-     * the persistent form runs lanes ahead of one another, so after a call
+     * the persistent form runs lanes ahead of one another (and its team form
+     * looks at a word every eighth iteration), so after a call
      * that lowered a word the caller restores the initial state and calls
      * again with the words as they were left.  NULL: every lane stops only
      * itself (per-lane semantics). */
