@@ -142,7 +142,7 @@ HYK_DM_FN int hyk_ev_narrow(const float *, int, float, int, float *, float *, fl
 
 /* Roots of q in (s_lo, s_hi] with direction dir (0: any, +1: dg/dt > 0,
  * -1: dg/dt < 0), in increasing order.  g: coefficients g_0..g_p at stride
- * gs; work: 3 (p + 1) numbers.  Stores at most maxr roots (rs[k * rstride]:
+ * gs; work: 2 (p + 1) numbers.  Stores at most maxr roots (rs[k * rstride]:
  * s, rsg[k * rstride]: direction) and returns how many roots it found, which
  * exceeds maxr when some were not stored; with first_only the walk stops at
  * the first root. */

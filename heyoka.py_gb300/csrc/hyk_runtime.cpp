@@ -405,6 +405,12 @@ static RegForm register_form(const hyk::Dec &d, uint32_t order, uint32_t flags, 
 // 41 s and 0.8 s).  The default form is kept unless another is estimated 5 %
 // faster, and of teams within 8 % of the fastest the one with the fewest
 // instructions is taken: the last trajectories then run fastest.
+//
+// The constants come from the systems above.  1000 trajectories of others, the form
+// taken and the best of all seven, ms: pendulum teams of 2 4.57 (4.57), Lorenz lane form
+// 1.50 (1.50), three bodies teams of 32 0.89 (of 16 0.78), six equations with
+// elementary functions teams of 4 3.40 (of 16 3.38), two powers of the time lane form
+// 0.54 (0.54).
 // (cold: with cold state rows where the system has them)
 static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool large, bool cold, size_t real_bytes,
                                const Device &dv, uint64_t n) {

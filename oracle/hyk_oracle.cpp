@@ -987,7 +987,7 @@ int propagate_ev(const Dec &d, uint32_t p, uint32_t B, double *state, const doub
     const uint32_t ne = d.n_eq, np = d.n_pars;
     std::vector<double> btd((size_t)(p + 1) * (p + 1));
     hyk_ev_btab((int)p, btd.data());
-    std::vector<T> bt(btd.begin(), btd.end()), work(3 * (p + 1)), g(p + 1);
+    std::vector<T> bt(btd.begin(), btd.end()), work(2 * (p + 1)), g(p + 1);
     const T cool_rel = sizeof(T) == sizeof(float) ? T(HYK_EV_COOL_REL_F) : T(HYK_EV_COOL_REL_D);
     uint32_t n_term = 0;
     std::vector<int> idx(d.ev.size());
@@ -1157,7 +1157,7 @@ int hyko_propagate_ev(const hyk_decomp_t *dd, uint32_t order, uint32_t B, double
 // The kernels' root finder on one polynomial (tests of hyk_events.h on the host).
 int hyko_ev_find(const double *g, uint32_t p, double h, double s_lo, double s_hi, int dir, int first_only, double *rs,
                  int32_t *rsg, int maxr) {
-    std::vector<double> bt((size_t)(p + 1) * (p + 1)), work(3 * (p + 1));
+    std::vector<double> bt((size_t)(p + 1) * (p + 1)), work(2 * (p + 1));
     hyk_ev_btab((int)p, bt.data());
     std::vector<int> sg(std::max(maxr, 1));
     const int n = hyk_ev_find<double>(g, 1, (int)p, h, bt.data(), s_lo, s_hi, dir, first_only, rs, sg.data(), 1, maxr,
