@@ -180,6 +180,11 @@ def _dev_index(device):
     return d.index if d.index is not None else torch.cuda.current_device()
 
 
+def _own_storage(t):
+    # (a row of an ensemble's stacked host tensors: pickled, it would carry them all)
+    return t.clone() if t.untyped_storage().nbytes() > t.numel() * t.element_size() else t
+
+
 def _two_sum(a, b):
     s = a + b
     bb = s - a
@@ -1400,7 +1405,7 @@ class taylor_adaptive_batch:
             if k in ("_mod", "_mod_grid"):
                 continue
             if isinstance(v, torch.Tensor):
-                d[k] = v.cpu()
+                d[k] = _own_storage(v.cpu())
             elif k == "_prop":
                 d[k] = None if v is None else {a: (None if b is None else b.cpu()) for a, b in v.items()}
             elif k == "_step_res":
