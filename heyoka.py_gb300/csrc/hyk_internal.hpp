@@ -63,6 +63,7 @@ struct TeamInfo {
     double util[6] = {0, 0, 0, 0, 0, 0};
     double instr[6] = {1, 1, 1, 1, 1, 1};  // FP64 instructions of a team's warp over those of one thread
     bool unrolled = false;  // the team form's orders in straight-line code
+    uint32_t n_shared = 0;  // values that four or more products read
     uint32_t n_spread[6] = {0, 0, 0, 0, 0, 0};  // doubles more for the powers' products spread over the team
     uint32_t n_raw = 0, n_raw_cold = 0;         // n_slot and n_slot_cold before the padding to an odd number
     // Doubles per trajectory of a team of T threads (odd).

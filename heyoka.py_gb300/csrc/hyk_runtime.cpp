@@ -395,24 +395,32 @@ static RegForm register_form(const hyk::Dec &d, uint32_t order, uint32_t flags, 
 // at work are counted at 0.7 of those at the start.  A small batch cannot fill
 // the warps of the lane form, so a team that spreads each trajectory wins
 // there.  Measured, us a step (estimated, in lane-form steps): 331 six-body
-// members with teams of 32 and 16 69 and 100 (0.089, 0.114), 3001 of them 249 and
-// 185 (0.195, 0.142); 1003 Kepler orbits in the lane form and with teams of 4
-// and 16 59, 42 and 39 (1.15, 0.77, 0.74), 10007 in the lane form and with teams
-// of 4 59 and 50 (1.15, 0.95); 1003 CR3BP trajectories in the lane form and with
-// teams of 16 96 and 86 (1.15, 1.06).  Lane-form systems so large that their recurrences are split into
-// functions and still spill are counted at c = 4 (first-order variational Kepler,
-// 42 equations: 2.05 ms a step in the lane form, 127 us with teams of 32; ptxas
-// 41 s and 0.8 s).  The default form is kept unless another is estimated 5 %
-// faster, and of teams within 8 % of the fastest the one with the fewest
-// instructions is taken: the last trajectories then run fastest.
+// members with teams of 32 and 16 69 and 100 (0.099, 0.123), 3001 of them 249 and
+// 185 (0.216, 0.152); 1003 Kepler orbits in the lane form and with teams of 4
+// and 16 59, 42 and 39 (1.15, 0.80, 0.74), 10007 in the lane form and with teams
+// of 4 59 and 50 (1.15, 0.99); 1003 CR3BP trajectories in the lane form and with
+// teams of 16 96 and 86 (1.15, 1.03).  The lane form of large systems, whose
+// recurrences are split into functions with the histories in memory, is counted at
+// c = 1.75, but at 8 where many values are read by four or more products each: the compiler
+// keeps such histories live over a whole order and spills (first-order variational Kepler,
+// 42 equations, twelve such values: 564 KB of spill stores, 3001 orbits 237 ms in the lane
+// form and 16 with teams of 16, 60013 270 and with teams of 8 74; ptxas 41 s and 0.8 s;
+// variational CR3BP, twenty values: 727 KB; Lorenz, three: 0; four bodies, none: 6 KB; 18
+// equations with elementary functions, none: 0), and at 4 where a team is the
+// default for full batches.  (At 4 for all, four bodies ran in teams of 8 at every
+// size: 250007 lanes 50.8 ms against 38.4 in the lane form, 60013 12.9 and 10.2, while 12007
+// take 3.2 and 5.6; 30011 of the 18 equations 10.0 against 8.1.)  The default form is kept unless another is estimated 4 %
+// faster (12007 Kepler orbits to t = 20 17.6 ms with teams of 4, 23.1 in the lane form; 4096 CR3BP
+// trajectories 3.07 and 3.22), and of the teams within 8 % of the fastest (and 2 % before the
+// default) the one with the fewest instructions is taken: the last trajectories then run fastest.
 //
 // The constants come from the systems above.  1000 trajectories of others, the form
 // taken and the best of all seven, ms: pendulum teams of 2 4.57 (4.57), Lorenz lane form
 // 1.50 (1.50), three bodies teams of 32 0.89 (of 16 0.78), six equations with
-// elementary functions teams of 4 3.40 (of 16 3.38), two powers of the time lane form
+// elementary functions teams of 8 (of 4 3.40, of 16 3.38), two powers of the time lane form
 // 0.54 (0.54).
 // (cold: with cold state rows where the system has them)
-static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool large, bool cold, size_t real_bytes,
+static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool large, bool spills, bool cold, size_t real_bytes,
                                const Device &dv, uint64_t n) {
     const double smsp = 4.0 * dv.n_sm;
     auto cost = [&](double c, double warps, double resident) {
@@ -421,7 +429,7 @@ static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool larg
         return t * std::max(1.0, w / std::max(k, 1e-9));
     };
     double c[6];
-    c[0] = cost(large ? 4.0 : 1.15, (double)n / 32.0, 2.0);
+    c[0] = cost(!large ? 1.15 : dflt ? 4.0 : spills ? 8.0 : 1.75, (double)n / 32.0, 2.0);
     for (uint32_t l = 1; l <= 5; ++l) {
         const uint32_t T = 1u << l;
         const size_t cta = (size_t)(32 / T) * team_slots(ti, T, cold, 32 / T, real_bytes, dv) * real_bytes;
@@ -434,10 +442,10 @@ static uint32_t team_for_batch(const hyk::TeamInfo &ti, uint32_t dflt, bool larg
     uint32_t best = 0;
     for (uint32_t l = 1; l <= 5; ++l)
         if (c[l] < c[best]) best = l;
-    if (c[best] * 1.05 >= c[dl]) return dflt;
+    if (c[best] * 1.04 >= c[dl]) return dflt;
     uint32_t pick = best;
     for (uint32_t l = 1; l <= 5; ++l)
-        if (best && c[l] <= 1.08 * c[best] && ti.instr[l] < 0.98 * ti.instr[pick]) pick = l;
+        if (best && c[l] <= 1.08 * c[best] && c[l] * 1.02 < c[dl] && ti.instr[l] < 0.98 * ti.instr[pick]) pick = l;
     return pick ? 1u << pick : 0;
 }
 
@@ -815,7 +823,8 @@ int hyk_config_for(const hyk_decomp_t *dd, uint32_t order, const hyk_config_t *c
     const uint32_t dflt = default_team(ti, lane_bytes, sizeof(double), *dv);
     const bool large = (uint64_t)d.n_ops * order > 3000 || lane_bytes * 32 > (size_t)dv->smem_optin;
     const bool cold = ti.n_slot_cold != 0 && !(c.flags & HYK_CFG_NO_COLD_ROWS);
-    const uint32_t team = team_for_batch(ti, dflt, large, cold, sizeof(double), *dv, n_lanes);
+    const bool spills = ti.n_shared * order > 127;  // (the doubles that 255 registers hold)
+    const uint32_t team = team_for_batch(ti, dflt, large, spills, cold, sizeof(double), *dv, n_lanes);
     if (team != dflt) c.team_size = team ? team : 1;
     // A team form whose trajectories are all resident at once without cold
     // state rows does without them (331 six-body members: teams of 32 87 us a
